@@ -46,10 +46,15 @@ def refdir() -> str:
     return os.environ.get("REFDIR") or os.path.normpath(os.path.join(HERE, os.pardir, os.pardir, "reference"))
 
 
+def have_sources() -> bool:
+    """Whether the reference checkout holds its sources (an empty directory does not)."""
+    return os.path.exists(os.path.join(refdir(), "src", "bhtree.cpp"))
+
+
 def build(reference: bool = True) -> None:
     """make -C oracle (the reference part only when its sources are present)."""
     targets = ["oracle"]
-    if reference and os.path.isdir(refdir()):
+    if reference and have_sources():
         targets.append("ref")
     subprocess.run(["make", "-s", "-C", HERE] + targets, check=True)
 
