@@ -118,6 +118,8 @@ struct sphgpu_ctx {
     // mixed-precision gravity: 32-byte FP32 node records of the current tree
     void* d_gnode = nullptr;
     int gnode_cap = 0;
+    // FP64 gravity: the particles' half kernels (gravity.cu)
+    double4* d_half = nullptr;
     bool have_mlp = false;
     std::vector<float> mlp_master;
     // pair-state harvesting (training data from the plain solver's own runs)
