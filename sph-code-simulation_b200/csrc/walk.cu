@@ -186,6 +186,16 @@ __device__ __forceinline__ double interval_gap(double c, double lo, double hi)
     return c < lo ? lo - c : (c > hi ? c - hi : 0.0);
 }
 
+// Periodic axis of length L, a group of extent ext, a candidate at offset b
+// (minimum image) from its centre.  A lane at offset a, |a| <= ext / 2, may
+// take d = a - b for the pair's offset when |d| <= L / 2 for sure; and else
+// when every image is further than h: then |d| > L / 2 > h, and the nearest
+// image is at least L / 2 - ext / 2 away.
+__device__ __forceinline__ bool image_safe(double b, double ext, double L, double h)
+{
+    return fabs(b) + 0.5 * ext < 0.499999 * L || 0.499999 * L - 0.5 * ext > h * (1.0 + 1e-6);
+}
+
 // exact box test of the reference's recursion at node nd for particle i
 template <bool IJ>
 __device__ __forceinline__ bool box_pass(const DevParams& P, const DevTree& T, int nd, double xi, double yi, double zi,
@@ -220,7 +230,6 @@ __global__ void __launch_bounds__(GW_WARPS * 32) k_walk_group(DevParams P, DevSt
     __shared__ float s_ctin[GW_WARPS][32];
     __shared__ int s_loff[GW_WARPS][32];
     __shared__ int s_lstart[GW_WARPS][32];
-    __shared__ double s_box[GW_WARPS][32][7];
     const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int i = (blockIdx.x * GW_WARPS + w) * 32 + lane;
     const bool valid = i < n;
@@ -244,47 +253,6 @@ __global__ void __launch_bounds__(GW_WARPS * 32) k_walk_group(DevParams P, DevSt
             hi = S.vel[i].w;
         }
     }
-    // Sub-groups.  A window of 32 octree-ordered particles that straddles a
-    // large octant boundary has a bounding box far wider than its particles'
-    // search spheres.  The warp is split into aligned sub-groups of s lanes
-    // (s = 32, 16, ..., 1: the largest s for which every sub-group's extent
-    // is at most GW_SPLIT times its largest radius) and the cooperative walk
-    // runs once per sub-group, all lanes traversing and staging, only the
-    // sub-group's lanes testing candidates.
-    const double own_lo[3] = {valid ? xi : 1e300, valid ? yi : 1e300, valid ? zi : 1e300};
-    const double own_up[3] = {valid ? xi : -1e300, valid ? yi : -1e300, valid ? zi : -1e300};
-    const double own_h = valid ? hi : 0.0;
-    int s = 1;
-    {
-        double l[3] = {own_lo[0], own_lo[1], own_lo[2]}, u[3] = {own_up[0], own_up[1], own_up[2]}, hm = own_h;
-        for(int o = 1; o < 32; o <<= 1) {
-            for(int k = 0; k < 3; ++k) {
-                l[k] = fmin(l[k], __shfl_xor_sync(FULL_MASK, l[k], o));
-                u[k] = fmax(u[k], __shfl_xor_sync(FULL_MASK, u[k], o));
-            }
-            hm = fmax(hm, __shfl_xor_sync(FULL_MASK, hm, o));
-            const double e = fmax(u[0] - l[0], fmax(u[1] - l[1], u[2] - l[2]));
-            if(__all_sync(FULL_MASK, e <= GW_SPLIT * hm)) s = 2 * o;
-        }
-    }
-    {
-        // each sub-group's box and radius, kept in shared memory
-        double lo[3] = {own_lo[0], own_lo[1], own_lo[2]}, up[3] = {own_up[0], own_up[1], own_up[2]};
-        double hmax = own_h;
-        for(int o = 1; o < s; o <<= 1) {
-            for(int k = 0; k < 3; ++k) {
-                lo[k] = fmin(lo[k], __shfl_xor_sync(FULL_MASK, lo[k], o));
-                up[k] = fmax(up[k], __shfl_xor_sync(FULL_MASK, up[k], o));
-            }
-            hmax = fmax(hmax, __shfl_xor_sync(FULL_MASK, hmax, o));
-        }
-        if(lane % s == 0) {
-            double* b = s_box[w][lane / s];
-            b[0] = lo[0], b[1] = lo[1], b[2] = lo[2], b[3] = up[0], b[4] = up[1], b[5] = up[2], b[6] = hmax;
-        }
-        __syncwarp();
-    }
-    if(lane == 0) atomicAdd(s == 32 ? &st->walk_group_warps : &st->walk_split_warps, 1ull);
     // safety margin for the fast acceptance (see above)
     const double4 root = ldg4(&T.geo[0]);
     const double scale = fmax(fabs(root.x), fmax(fabs(root.y), fabs(root.z))) + root.w;
@@ -293,12 +261,54 @@ __global__ void __launch_bounds__(GW_WARPS * 32) k_walk_group(DevParams P, DevSt
     const size_t row = (size_t)(valid ? i : 0) * (size_t)cap;
     int cnt = 0;
     bool overflow = false;
-    for(int sg = 0; sg < 32 / s && !overflow; ++sg) {
-        const bool act = valid && lane / s == sg;
+    // Sub-groups.  A window of 32 octree-ordered particles that straddles a
+    // large octant boundary has a bounding box far wider than its particles'
+    // search spheres.  The warp takes runs of lanes whose extent is at most
+    // GW_SPLIT times their largest radius, from the first lane on, each run up
+    // to the jump that breaks it, and walks once per run: all lanes traverse
+    // and stage, the run's lanes test candidates.  (Halving the window until
+    // every aligned part fits put all 32 lanes of a window whose jump lies at
+    // an odd lane into walks of their own: with few warps those were the
+    // kernel's tail, 17 K sphere 0.49 ms against 0.14.)
+    int first = 0;
+    while(first < 32 && !overflow) {
+        const bool in = valid && lane >= first;
+        double blo[3] = {in ? xi : 1e300, in ? yi : 1e300, in ? zi : 1e300};
+        double bup[3] = {in ? xi : -1e300, in ? yi : -1e300, in ? zi : -1e300};
+        double bh = in ? hi : 0.0;
+        for(int o = 1; o < 32; o <<= 1) {
+            // the box of lanes first .. this one
+            const bool take = lane - o >= first;
+            for(int k = 0; k < 3; ++k) {
+                const double l = __shfl_up_sync(FULL_MASK, blo[k], o), u = __shfl_up_sync(FULL_MASK, bup[k], o);
+                if(take) {
+                    blo[k] = fmin(blo[k], l);
+                    bup[k] = fmax(bup[k], u);
+                }
+            }
+            const double m = __shfl_up_sync(FULL_MASK, bh, o);
+            if(take) bh = fmax(bh, m);
+        }
+        bool fits = true;
+        for(int k = 0; k < 3; ++k) {
+            const double ext = bup[k] - blo[k];
+            fits = fits && ext <= GW_SPLIT * bh;
+            // a periodic axis: extents for which image_safe holds everywhere,
+            // unless the box is too short for any
+            const double most = P.range[k] - 2.02 * bh;
+            if(P.periodic && most > 0.0) fits = fits && ext < most;
+        }
+        const unsigned far = __ballot_sync(FULL_MASK, in && lane > first && !fits);
+        const int last = far ? __ffs(far) - 2 : 31;
+        for(int k = 0; k < 3; ++k) {
+            blo[k] = __shfl_sync(FULL_MASK, blo[k], last);
+            bup[k] = __shfl_sync(FULL_MASK, bup[k], last);
+        }
+        bh = __shfl_sync(FULL_MASK, bh, last);
+        const bool act = in && lane <= last;
+        if(lane == 0 && first == 0) atomicAdd(far ? &st->walk_split_warps : &st->walk_group_warps, 1ull);
+        first = last + 1;
         if(__ballot_sync(FULL_MASK, act) == 0) continue;
-        const double* bb = s_box[w][sg];
-        const double blo[3] = {bb[0], bb[1], bb[2]}, bup[3] = {bb[3], bb[4], bb[5]};
-        const double bh = bb[6];
         const double bext = fmax(bup[0] - blo[0], fmax(bup[1] - blo[1], bup[2] - blo[2]));
         int sp = 0, nq = 0;
         if(lane == 0) s_stack[w][0] = 0;
@@ -319,8 +329,10 @@ __global__ void __launch_bounds__(GW_WARPS * 32) k_walk_group(DevParams P, DevSt
         // so it is taken without FP64 work; only pairs between the thresholds run
         // the exact FP64 test.  With periodic wrapping the FP32 offset is the
         // minimum image only if |b_j| + ext/2 < L/2 on every axis (|a_i| <= ext/2);
-        // other candidates are staged with NaN offsets and always run the exact
-        // test.  Each lane classifies a chunk of 32 staged candidates branch-free
+        // and an offset that is not it is certainly outside where image_safe
+        // holds; other candidates are staged with NaN offsets and always run the
+        // exact test (2.3 us a candidate: without image_safe's second case most
+        // candidates of a thin periodic box took it, 245 K tube 1.44 ms).  Each lane classifies a chunk of 32 staged candidates branch-free
         // into two bit masks (inside, band), runs the exact test for the band
         // bits and writes the taken candidates in chunk order.
         const double cx = 0.5 * (blo[0] + bup[0]), cy = 0.5 * (blo[1] + bup[1]), cz = 0.5 * (blo[2] + bup[2]);
@@ -373,9 +385,11 @@ __global__ void __launch_bounds__(GW_WARPS * 32) k_walk_group(DevParams P, DevSt
                         bx = min_image(bx, P.range[0]);
                         by = min_image(by, P.range[1]);
                         bz = min_image(bz, P.range[2]);
-                        pre = fabs(bx) + 0.5 * ext_x < 0.499999 * P.range[0]
-                            && fabs(by) + 0.5 * ext_y < 0.499999 * P.range[1]
-                            && fabs(bz) + 0.5 * ext_z < 0.499999 * P.range[2];
+                        // the offset is the minimum image for every lane, or the
+                        // axis alone keeps the pair apart either way round
+                        const double hk = IJ ? fmax(bh, ks) : bh;
+                        pre = image_safe(bx, ext_x, P.range[0], hk) && image_safe(by, ext_y, P.range[1], hk)
+                            && image_safe(bz, ext_z, P.range[2], hk);
                     }
                     float tko = -1.0f, tki = -1.0f;
                     if(IJ) {
