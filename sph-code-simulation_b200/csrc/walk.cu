@@ -181,6 +181,32 @@ constexpr int GW_QUEUE = 64;
 constexpr int GW_WHOLE = 8;   // nodes with at most this many particles are queued whole
 constexpr double GW_SPLIT = 6.0;  // sub-group extent limit, in units of its largest radius
 
+// Two FP32 values in a 64-bit register, and the packed operations on them
+// (rounded to nearest, like the scalar ones): half the issue slots.
+using f32x2 = unsigned long long;
+__device__ __forceinline__ f32x2 pack2(float a, float b)
+{
+    f32x2 r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+    return r;
+}
+__device__ __forceinline__ f32x2 add2(f32x2 a, f32x2 b)
+{
+    f32x2 r;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c)
+{
+    f32x2 r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+    return r;
+}
+__device__ __forceinline__ unsigned lo32(f32x2 a) { return (unsigned)a; }
+__device__ __forceinline__ unsigned hi32(f32x2 a) { return (unsigned)(a >> 32); }
+// mask << 1 | sign bit of v
+__device__ __forceinline__ unsigned sign_in(unsigned mask, unsigned v) { return __funnelshift_l(v, mask, 1); }
+
 __device__ __forceinline__ double interval_gap(double c, double lo, double hi)
 {
     return c < lo ? lo - c : (c > hi ? c - hi : 0.0);
@@ -216,20 +242,23 @@ __device__ __forceinline__ bool box_pass(const DevParams& P, const DevTree& T, i
     return m <= l2;
 }
 
-template <bool IJ>
-__global__ void __launch_bounds__(GW_WARPS * 32) k_walk_group(DevParams P, DevState S, DevTree T, int n, int cap,
+// RES: resident blocks per SM (caps the registers).  9 (112 registers) where
+// the launch fills the chip: 1 M shear 2.98 -> 2.82 ms, 2 M tube 3.42 -> 3.22;
+// 8 (128 registers) where a warp's own latency counts: 137 K sphere 0.93 ->
+// 0.81, 17 K 0.215 -> 0.185.  The line is about four rounds of blocks.
+constexpr int GW_FEW = 148 * 8 * GW_WARPS * 32 * 4;
+template <bool IJ, int RES>
+__global__ void __launch_bounds__(GW_WARPS * 32, RES) k_walk_group(DevParams P, DevState S, DevTree T, int n, int cap,
                                                              int* __restrict__ list, int* __restrict__ count,
                                                              DevStatus* __restrict__ st, int guess, double ratio,
                                                              SkinOut sk)
 {
     __shared__ int s_stack[GW_WARPS][GW_STACK];
     __shared__ int s_queue[GW_WARPS][GW_QUEUE];
-    __shared__ float4 s_cf[GW_WARPS][32];
+    __shared__ __align__(16) float s_cx[GW_WARPS][32], s_cy[GW_WARPS][32], s_cz[GW_WARPS][32];
     __shared__ double4 s_cpos[GW_WARPS][32];
-    __shared__ int s_cid[GW_WARPS][32];
-    __shared__ float s_ctin[GW_WARPS][32];
-    __shared__ int s_loff[GW_WARPS][32];
-    __shared__ int s_lstart[GW_WARPS][32];
+    __shared__ __align__(16) int s_cid[GW_WARPS][32];
+    __shared__ float2 s_ct[GW_WARPS][IJ ? 32 : 1];
     const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int i = (blockIdx.x * GW_WARPS + w) * 32 + lane;
     const bool valid = i < n;
@@ -258,8 +287,9 @@ __global__ void __launch_bounds__(GW_WARPS * 32) k_walk_group(DevParams P, DevSt
     const double scale = fmax(fabs(root.x), fmax(fabs(root.y), fabs(root.z))) + root.w;
     const double delta = 1e-12 * scale;
 
-    const size_t row = (size_t)(valid ? i : 0) * (size_t)cap;
+    int* out = list + (size_t)(valid ? i : 0) * (size_t)cap;
     int cnt = 0;
+    int4 four = make_int4(0, 0, 0, 0);  // the last entries taken
     bool overflow = false;
     // Sub-groups.  A window of 32 octree-ordered particles that straddles a
     // large octant boundary has a bounding box far wider than its particles'
@@ -268,8 +298,8 @@ __global__ void __launch_bounds__(GW_WARPS * 32) k_walk_group(DevParams P, DevSt
     // to the jump that breaks it, and walks once per run: all lanes traverse
     // and stage, the run's lanes test candidates.  (Halving the window until
     // every aligned part fits put all 32 lanes of a window whose jump lies at
-    // an odd lane into walks of their own: with few warps those were the
-    // kernel's tail, 17 K sphere 0.49 ms against 0.14.)
+    // an odd lane into walks of their own, the kernel's tail: 17 K sphere 0.385
+    // -> 0.245 ms, 2 M tube 4.94 -> 3.86.)
     int first = 0;
     while(first < 32 && !overflow) {
         const bool in = valid && lane >= first;
@@ -329,12 +359,17 @@ __global__ void __launch_bounds__(GW_WARPS * 32) k_walk_group(DevParams P, DevSt
         // so it is taken without FP64 work; only pairs between the thresholds run
         // the exact FP64 test.  With periodic wrapping the FP32 offset is the
         // minimum image only if |b_j| + ext/2 < L/2 on every axis (|a_i| <= ext/2);
-        // and an offset that is not it is certainly outside where image_safe
-        // holds; other candidates are staged with NaN offsets and always run the
-        // exact test (2.3 us a candidate: without image_safe's second case most
-        // candidates of a thin periodic box took it, 245 K tube 1.44 ms).  Each lane classifies a chunk of 32 staged candidates branch-free
-        // into two bit masks (inside, band), runs the exact test for the band
-        // bits and writes the taken candidates in chunk order.
+        // and where it is not, the pair is certainly outside either way if
+        // image_safe holds; other candidates always run the exact test (most of
+        // a thin periodic box's did without image_safe's second case: 131 K shear
+        // layer 1.31 -> 0.63 ms, 245 K tube 1.44 -> 0.69).
+        // Each lane classifies a chunk of 32 staged candidates branch-free into
+        // two bit masks (inside, band), runs the exact test for the band bits and
+        // writes the taken candidates in chunk order.  Issue-bound (1 M shear: 60 K
+        // instructions a warp for 59 chunks, 61 % of the issue slots): two
+        // candidates per packed FP32 operation, each mask bit one funnel shift of a
+        // sign, the candidates' nodes found by ballots, the next chunk's positions
+        // in flight (3.33 -> 2.82 ms; scalar FP32 3.01).
         const double cx = 0.5 * (blo[0] + bup[0]), cy = 0.5 * (blo[1] + bup[1]), cz = 0.5 * (blo[2] + bup[2]);
         const double ext_x = bup[0] - blo[0], ext_y = bup[1] - blo[1], ext_z = bup[2] - blo[2];
         const float ax = (float)(xi - cx), ay = (float)(yi - cy), az = (float)(zi - cz);
@@ -344,10 +379,21 @@ __global__ void __launch_bounds__(GW_WARPS * 32) k_walk_group(DevParams P, DevSt
         };
         auto t_in = [&](double h) -> float {
             const double t = (h - delta - (0x1p-22 * bext + 0x1p-21 * h)) * (1.0 - 0x1p-20);
-            return t > 0.0 ? __double2float_rd(t * t * (1.0 - 0x1p-20)) : -1.0f;
+            // (a radius below about 2^-20 of the extent: band pairs only, so that
+            // Tout < 2 t^2 wherever a pair may be taken without the exact test)
+            const double o = h * (1.0 + 0x1p-20) + 0x1p-21 * bext;
+            return t > 0.0 && o * o < 1.9 * (t * t) ? __double2float_rd(t * t * (1.0 - 0x1p-20)) : -1.0f;
         };
         const float Ti_out = act ? t_out(hi) : -1.0f;
         const float Ti_in = act ? t_in(hi) : -1.0f;
+        // The gather walk's tests as signs: s = r2f - Tout and s + (Tout - Tin),
+        // accumulated with FMA.  With S the exact sum of squares of the FP32
+        // offsets, s is within 3 * 2^-24 max(Tout, S) of S - Tout and the second
+        // within 4 * 2^-24 Tout more: inside the 2^-20 that the thresholds leave.
+        const f32x2 A2x = pack2(ax, ax), A2y = pack2(ay, ay), A2z = pack2(az, az);
+        const f32x2 O2 = pack2(-Ti_out, -Ti_out);
+        const float gap = Ti_out - Ti_in;
+        const f32x2 G2 = pack2(gap, gap);
         const float F_INF = __int_as_float(0x7f800000);
         const float F_NAN = __int_as_float(0x7fffffff);
 
@@ -365,22 +411,28 @@ __global__ void __launch_bounds__(GW_WARPS * 32) k_walk_group(DevParams P, DevSt
                 if(lane >= o) incl += u;
             }
             const int total = __shfl_sync(FULL_MASK, incl, 31);
-            s_loff[w][lane] = incl - lcnt;
-            s_lstart[w][lane] = lstart;
-            __syncwarp();
+            const int excl = incl - lcnt, shift = lstart - excl;
+            // candidate g of the queue: in the last node t with excl_t <= g
+            auto candidate = [&](int base) {
+                const unsigned before = __ballot_sync(FULL_MASK, lane < nproc && excl <= base);
+                const bool starts = lane < nproc && excl > base && excl < base + 32;
+                const unsigned marks = __reduce_or_sync(FULL_MASK, starts ? 1u << (excl - base) : 0u);
+                const int t = __popc(before) - 1 + __popc(marks & ((2u << lane) - 1u));
+                return __shfl_sync(FULL_MASK, shift, t & 31) + base + lane;
+            };
+            // the next chunk's positions are loaded while this one is classified
+            int qn = candidate(0);
+            double4 pn = lane < total ? ldg4(&S.pos[qn]) : make_double4(0, 0, 0, 0);
             for(int base = 0; base < total; base += 32) {
-                const int g = base + lane;
-                if(g < total) {
-                    // the leaf holding candidate g: largest t < nproc with loff[t] <= g
-                    int t = 0;
-                    for(int s = 16; s > 0; s >>= 1) {
-                        if(t + s < nproc && s_loff[w][t + s] <= g) t += s;
-                    }
-                    const int q = s_lstart[w][t] + (g - s_loff[w][t]);
-                    const double4 pj = ldg4(&S.pos[q]);
+                const bool have = base + lane < total;
+                const int q = qn;
+                const double4 pj = pn;
+                bool pre = true;
+                float fx = F_INF, fy = F_INF, fz = F_INF;  // padding: infinitely far, never taken
+                float tko = -1.0f, tki = -1.0f;
+                if(have) {
                     const double ks = IJ ? __ldg(&T.pks[q]) : 0.0;
                     double bx = xsub(pj.x, cx), by = xsub(pj.y, cy), bz = xsub(pj.z, cz);
-                    bool pre = true;
                     if(P.periodic) {
                         bx = min_image(bx, P.range[0]);
                         by = min_image(by, P.range[1]);
@@ -391,45 +443,77 @@ __global__ void __launch_bounds__(GW_WARPS * 32) k_walk_group(DevParams P, DevSt
                         pre = image_safe(bx, ext_x, P.range[0], hk) && image_safe(by, ext_y, P.range[1], hk)
                             && image_safe(bz, ext_z, P.range[2], hk);
                     }
-                    float tko = -1.0f, tki = -1.0f;
                     if(IJ) {
                         tko = t_out(ks);
                         tki = t_in(ks);
                     }
-                    float fx = (float)bx, fy = (float)by, fz = (float)bz;
-                    if(!pre) fx = fy = fz = F_NAN;  // classified as band: exact test
-                    s_cf[w][lane] = make_float4(fx, fy, fz, tko);
-                    s_ctin[w][lane] = tki;
+                    fx = (float)bx;
+                    fy = (float)by;
+                    fz = (float)bz;
                     s_cpos[w][lane] = make_double4(pj.x, pj.y, pj.z, ks);
                     s_cid[w][lane] = q;
-                } else {
-                    // padding: infinitely far, never taken
-                    s_cf[w][lane] = make_float4(F_INF, F_INF, F_INF, -1.0f);
-                    s_ctin[w][lane] = -1.0f;
+                }
+                // candidates whose image depends on the lane: exact tests
+                const unsigned force = __ballot_sync(FULL_MASK, !pre);
+                s_cx[w][lane] = -fx;
+                s_cy[w][lane] = -fy;
+                s_cz[w][lane] = -fz;
+                if(IJ) s_ct[w][lane] = make_float2(tko, tki);
+                if(base + 32 < total) {
+                    qn = candidate(base + 32);
+                    if(base + 32 + lane < total) pn = ldg4(&S.pos[qn]);
                 }
                 __syncwarp();
+                unsigned in_mask = 0u;
                 if(act) {
-                    unsigned in_mask = 0u, band_mask = 0u;
-    #pragma unroll
-                    for(int k = 0; k < 32; ++k) {
-                        const float4 b = s_cf[w][k];
-                        const float dx = ax - b.x, dy = ay - b.y, dz = az - b.z;
-                        const float r2f = fmaf(dz, dz, fmaf(dy, dy, dx * dx));
-                        const float to = IJ ? fmaxf(Ti_out, b.w) : Ti_out;
-                        const float ti = IJ ? fmaxf(Ti_in, s_ctin[w][k]) : Ti_in;
-                        const bool inside = r2f < ti;
-                        const bool band = !inside && !(r2f >= to);  // NaN offsets land here
-                        in_mask |= (unsigned)inside << k;
-                        band_mask |= (unsigned)band << k;
+                    unsigned band_mask = 0u;
+                    if constexpr(!IJ) {
+                        unsigned near = 0u, inside = 0u;
+#pragma unroll
+                        for(int k = 28; k >= 0; k -= 4) {
+                            const ulonglong2 X = *reinterpret_cast<const ulonglong2*>(&s_cx[w][k]);
+                            const ulonglong2 Y = *reinterpret_cast<const ulonglong2*>(&s_cy[w][k]);
+                            const ulonglong2 Z = *reinterpret_cast<const ulonglong2*>(&s_cz[w][k]);
+                            const f32x2 xa = add2(A2x, X.x), ya = add2(A2y, Y.x), za = add2(A2z, Z.x);
+                            const f32x2 xb = add2(A2x, X.y), yb = add2(A2y, Y.y), zb = add2(A2z, Z.y);
+                            const f32x2 sa = fma2(za, za, fma2(ya, ya, fma2(xa, xa, O2)));
+                            const f32x2 sb = fma2(zb, zb, fma2(yb, yb, fma2(xb, xb, O2)));
+                            const f32x2 ta = add2(sa, G2), tb = add2(sb, G2);
+                            near = sign_in(near, hi32(sb));
+                            near = sign_in(near, lo32(sb));
+                            near = sign_in(near, hi32(sa));
+                            near = sign_in(near, lo32(sa));
+                            inside = sign_in(inside, hi32(tb));
+                            inside = sign_in(inside, lo32(tb));
+                            inside = sign_in(inside, hi32(ta));
+                            inside = sign_in(inside, lo32(ta));
+                        }
+                        in_mask = inside & ~force;
+                        band_mask = (near & ~inside) | force;
+                    } else {
+#pragma unroll
+                        for(int k = 0; k < 32; ++k) {
+                            const float dx = ax + s_cx[w][k], dy = ay + s_cy[w][k], dz = az + s_cz[w][k];
+                            const float2 tk = s_ct[w][k];
+                            const float r2f = fmaf(dz, dz, fmaf(dy, dy, dx * dx));
+                            const float to = fmaxf(Ti_out, tk.x);
+                            const float ti = fmaxf(Ti_in, tk.y);
+                            const bool inside = r2f < ti;
+                            const bool band = !inside && !(r2f >= to);
+                            in_mask |= (unsigned)inside << k;
+                            band_mask |= (unsigned)band << k;
+                        }
+                        in_mask &= ~force;
+                        band_mask |= force;
                     }
                     while(band_mask) {
                         const int k = __ffs(band_mask) - 1;
                         band_mask &= band_mask - 1u;
-                        const int q = s_cid[w][k];
-                        const double4 pj = s_cpos[w][k];
+                        const int qk = s_cid[w][k];
+                        const double4 pk = s_cpos[w][k];
                         double h = hi;
-                        if(IJ) h = hi < pj.w ? pj.w : hi;
-                        const Vec3d r = rij(P, xi, yi, zi, pj.x, pj.y, pj.z);
+                        if(IJ) h = hi < pk.w ? pk.w : hi;
+                        const Vec3d r = rij(P, xi, yi, zi, pk.x, pk.y, pk.z);
                         const double r2 = abs2x(r);
                         if(!(r2 < h * h)) continue;
                         const double hs = h - delta;
@@ -437,7 +521,7 @@ __global__ void __launch_bounds__(GW_WARPS * 32) k_walk_group(DevParams P, DevSt
                         if(!take) {
                             // on the radius: replay the reference's box tests up the path
                             take = true;
-                            int A = __ldg(&T.leaf_of[q]);
+                            int A = __ldg(&T.leaf_of[qk]);
                             for(int up_ = 0; A >= 0 && up_ < 64; ++up_) {
                                 if(!box_pass<IJ>(P, T, A, xi, yi, zi, hi)) {
                                     take = false;
@@ -448,12 +532,18 @@ __global__ void __launch_bounds__(GW_WARPS * 32) k_walk_group(DevParams P, DevSt
                         }
                         if(take) in_mask |= 1u << k;
                     }
-                    while(in_mask) {
-                        const int k = __ffs(in_mask) - 1;
-                        in_mask &= in_mask - 1u;
-                        if(cnt < cap) list[row + cnt] = s_cid[w][k];
-                        ++cnt;
-                    }
+                }
+                // Every lane appends its entries, four to a 16-byte store (rows
+                // start on 128 bytes): a store of single entries goes to 32
+                // rows at once.
+                while(in_mask) {
+                    const int k = __ffs(in_mask) - 1;
+                    in_mask &= in_mask - 1u;
+                    four.x = four.y;
+                    four.y = four.z;
+                    four.z = four.w;
+                    four.w = s_cid[w][k];
+                    if((++cnt & 3) == 0 && cnt <= cap) *reinterpret_cast<int4*>(out + cnt - 4) = four;
                 }
                 __syncwarp();
             }
@@ -547,11 +637,19 @@ __global__ void __launch_bounds__(GW_WARPS * 32) k_walk_group(DevParams P, DevSt
         return;
     }
     if(valid) {
+        // the entries past the last whole four
+        const int rem = cnt & 3;
+        if(cnt <= cap) {
+            if(rem == 3) out[cnt - 3] = four.y;
+            if(rem >= 2) out[cnt - 2] = four.z;
+            if(rem >= 1) out[cnt - 1] = four.w;
+        }
         count[i] = cnt;
         if(cnt > cap) st->overflow = 1;
         if(cnt > P.nngb * 1000) st->fatal = 1;
-        atomicMax(&st->max_count, cnt);
     }
+    const int longest = __reduce_max_sync(FULL_MASK, valid ? cnt : 0);
+    if(lane == 0) atomicMax(&st->max_count, longest);
 }
 
 // exhaustive_search (src/exhaustive_search.cpp:11-42): all j with
@@ -621,12 +719,15 @@ int run_walk(sphgpu_ctx* c, int which, bool guess, double ratio, bool exhaustive
             k_exhaustive<<<grid_for(n, 128), 128, 0, st>>>(c->dp, c->s, n, is_ij, (int)cap, list, count, c->d_status);
         } else if(c->walk_mode == 0 && !per_lane) {
             const unsigned grid = grid_for(n, GW_WARPS * 32);
+            const bool few = n <= GW_FEW;
             if(which == 0) {
-                k_walk_group<false><<<grid, GW_WARPS * 32, 0, st>>>(c->dp, c->s, c->t, n, (int)cap, list, count,
-                                                                   c->d_status, guess ? 1 : 0, ratio, sk);
+                auto* k = few ? k_walk_group<false, 8> : k_walk_group<false, 9>;
+                k<<<grid, GW_WARPS * 32, 0, st>>>(c->dp, c->s, c->t, n, (int)cap, list, count, c->d_status,
+                                                  guess ? 1 : 0, ratio, sk);
             } else {
-                k_walk_group<true><<<grid, GW_WARPS * 32, 0, st>>>(c->dp, c->s, c->t, n, (int)cap, list, count,
-                                                                  c->d_status, 0, 1.0, SkinOut{1.0, nullptr, nullptr});
+                auto* k = few ? k_walk_group<true, 8> : k_walk_group<true, 9>;
+                k<<<grid, GW_WARPS * 32, 0, st>>>(c->dp, c->s, c->t, n, (int)cap, list, count, c->d_status, 0, 1.0,
+                                                  SkinOut{1.0, nullptr, nullptr});
             }
         } else if(which == 0) {
             k_walk<false><<<grid_for(n, WBLK), WBLK, 0, st>>>(c->dp, c->s, c->t, n, (int)cap, list, count,
