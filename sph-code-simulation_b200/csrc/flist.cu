@@ -117,34 +117,80 @@ __global__ void __launch_bounds__(LBLK, 5) k_flist(DevParams P, DevState S, int 
     }
 }
 
-// Appended entries: sorted by index and moved behind the own entries.
-__global__ void k_flist_finalize(int n, int* __restrict__ plist, int* __restrict__ pcount,
-                                 const int* __restrict__ tcount, int pcap, int fatal_limit,
-                                 int* __restrict__ flags)
+// Appended entries: sorted by index and moved behind the own entries.  A warp
+// takes 32 rows: a few entries are sorted by the row's own lane, longer tails
+// by the whole warp, every entry to its rank (indices are unique).  In a
+// graded sphere the centre's rows are appended to by a hundred neighbours and
+// more; one lane's insertion sort over global memory was then the pass.
+constexpr int FSHORT = 4;      // entries a lane sorts by itself, in registers
+constexpr int FBUF = 512;      // entries a warp ranks from shared memory
+constexpr int FWARPS = 4;
+__global__ void __launch_bounds__(FWARPS * 32) k_flist_finalize(int n, int* __restrict__ plist,
+                                                               int* __restrict__ pcount,
+                                                               const int* __restrict__ tcount, int pcap,
+                                                               int fatal_limit, int* __restrict__ flags)
 {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if(i >= n) return;
-    const int oc = pcount[i], tc = tcount[i];
+    __shared__ int s_buf[FWARPS][FBUF];
+    const int lane = threadIdx.x & 31;
+    int* buf = s_buf[threadIdx.x >> 5];
+    const int i = blockIdx.x * FWARPS * 32 + threadIdx.x;
+    const bool valid = i < n;
+    const int oc = valid ? pcount[i] : 0, tc = valid ? tcount[i] : 0;
     const long long tot = (long long)oc + tc;
-    if(tot > pcap) {
-        flags[0] = 1;
-        return;
-    }
-    if(tot > fatal_limit) flags[2] = 1;
-    int* row = plist + (size_t)i * (size_t)pcap;
-    const int b0 = pcap - tc;
-    for(int a = b0 + 1; a < pcap; ++a) {
-        const int v = row[a];
-        int b = a - 1;
-        while(b >= b0 && row[b] > v) {
-            row[b + 1] = row[b];
-            --b;
+    const bool fits = tot <= pcap;
+    if(!fits) flags[0] = 1;
+    if(fits && tot > fatal_limit) flags[2] = 1;
+    int* row = plist + (size_t)(valid ? i : 0) * (size_t)pcap;
+    if(fits && tc > 0 && tc <= FSHORT) {
+        int v[FSHORT];
+#pragma unroll
+        for(int t = 0; t < FSHORT; ++t) v[t] = t < tc ? row[pcap - 1 - t] : 0x7fffffff;
+#pragma unroll
+        for(int t = 0; t < FSHORT; ++t) {
+            int rank = 0;
+#pragma unroll
+            for(int u = 0; u < FSHORT; ++u) rank += v[u] < v[t] ? 1 : 0;
+            if(t < tc) row[oc + rank] = v[t];
         }
-        row[b + 1] = v;
     }
-    for(int t = 0; t < tc; ++t) row[oc + t] = row[b0 + t];
-    pcount[i] = (int)tot;
-    atomicMax(&flags[1], (int)tot);
+    for(unsigned left = __ballot_sync(FULL_MASK, fits && tc > FSHORT); left; left &= left - 1u) {
+        const int L = __ffs(left) - 1;
+        const int c = __shfl_sync(FULL_MASK, tc, L), o = __shfl_sync(FULL_MASK, oc, L);
+        int* r = plist + (size_t)(i - lane + L) * (size_t)pcap;
+        const int* tail = r + (pcap - c);
+        if(c <= 32) {
+            const int v = lane < c ? tail[lane] : 0x7fffffff;
+            int rank = 0;
+            for(int t = 0; t < c; ++t) rank += __shfl_sync(FULL_MASK, v, t) < v ? 1 : 0;
+            if(lane < c) r[o + rank] = v;
+        } else if(c <= FBUF) {
+            // the whole tail is read before its place is written over
+            for(int t = lane; t < c; t += 32) buf[t] = tail[t];
+            __syncwarp();
+            for(int t = lane; t < c; t += 32) {
+                const int v = buf[t];
+                int rank = 0;
+                for(int u = 0; u < c; ++u) rank += buf[u] < v ? 1 : 0;
+                r[o + rank] = v;
+            }
+            __syncwarp();
+        } else if(lane == 0) {
+            int* t = r + (pcap - c);
+            for(int a = 1; a < c; ++a) {
+                const int v = t[a];
+                int b = a - 1;
+                while(b >= 0 && t[b] > v) {
+                    t[b + 1] = t[b];
+                    --b;
+                }
+                t[b + 1] = v;
+            }
+            for(int a = 0; a < c; ++a) r[o + a] = t[a];
+        }
+    }
+    if(fits && valid) pcount[i] = (int)tot;
+    const int longest = __reduce_max_sync(FULL_MASK, fits ? (int)tot : 0);
+    if(lane == 0 && longest > 0) atomicMax(&flags[1], longest);
 }
 
 }  // namespace
@@ -168,7 +214,7 @@ int build_force_lists(sphgpu_ctx* c)
     k_flist<LG><<<grid, LBLK, 0, st>>>(c->dp, c->s, n, c->d_glist, c->d_gcount, (int)c->gcap, c->d_rsearch,
                                        c->d_plist, c->d_pcount, c->d_tcount, (int)c->pcap, c->d_flist_flags,
                                        c->t, c->skin_valid ? c->skin_delta_now : 0.0);
-    k_flist_finalize<<<grid_for(n, 256), 256, 0, st>>>(n, c->d_plist, c->d_pcount, c->d_tcount, (int)c->pcap,
+    k_flist_finalize<<<grid_for(n, FWARPS * 32), FWARPS * 32, 0, st>>>(n, c->d_plist, c->d_pcount, c->d_tcount, (int)c->pcap,
                                                         c->prm.neighbor_number * 1000, c->d_flist_flags);
     SPHGPU_LAUNCH_CHECK(c, "force lists");
     stage_end(c, SPHGPU_T_PAIR_WALK, 2);
