@@ -39,6 +39,7 @@ int check_pass_guard(sphgpu_ctx* c)
     if(bits & PASS_GUARD_KSIZE) m += " set_kernel";
     if(bits & PASS_GUARD_GRAVITY) m += " gravity walk";
     if(bits & PASS_GUARD_GRAVITY32) m += " mixed gravity walk";
+    if(bits & PASS_GUARD_SORT) m += " key sort (a wait for an earlier tile)";
     return fail(c, SPHGPU_ERR_STATE, m);
 }
 

@@ -137,6 +137,7 @@ constexpr int PASS_GUARD_MASS = 1;       // bottom-up mass / centre of mass
 constexpr int PASS_GUARD_KSIZE = 2;      // bottom-up kernel_size (set_kernel)
 constexpr int PASS_GUARD_GRAVITY = 4;    // Barnes-Hut walk (FP64)
 constexpr int PASS_GUARD_GRAVITY32 = 8;  // Barnes-Hut walk (mixed form)
+constexpr int PASS_GUARD_SORT = 16;      // look-back of a radix sort pass
 
 // Read-only 32-byte load through the non-coherent path, one 256-bit access
 // (sm_100).  p must be 32-byte aligned: every double4 array here is an

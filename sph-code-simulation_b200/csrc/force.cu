@@ -660,10 +660,10 @@ __global__ void k_iota(uint32_t* v, int n)
 
 // Per particle, the first sorted row and the number of rows of its deferred pairs.
 __global__ void k_defer_ranges(const uint64_t* __restrict__ skeys, int n, uint64_t cap, int* __restrict__ dstart,
-                               int* __restrict__ dcount)
+                               int* __restrict__ dcount, const DevStatus* __restrict__ st)
 {
     const int r = blockIdx.x * blockDim.x + threadIdx.x;
-    if(r >= n) return;
+    if(r >= n || (st->pass_guard & PASS_GUARD_SORT)) return;  // (rows not sorted: the host reports it)
     const uint64_t p = skeys[r] / cap;
     if(r == 0 || skeys[r - 1] / cap != p) dstart[p] = r;
     atomicAdd(&dcount[p], 1);
@@ -740,9 +740,11 @@ int fluid_force(sphgpu_ctx* c)
             while(bits < 32 && (1ull << bits) < (unsigned long long)slots) ++bits;
             uint64_t *kk = L.keys, *ka = L.keys_alt;
             uint32_t *vv = L.vals, *va = L.vals_alt;
-            launches += 2 + radix_sort(kk, vv, ka, va, nr, (bits + 7) / 8 * 8, L.scratch, c->stream);
+            launches += 2 + radix_sort(kk, vv, ka, va, nr, (bits + 7) / 8 * 8, L.scratch,
+                                         &c->d_status->pass_guard, c->stream);
             SPHGPU_CUDA(c, cudaMemsetAsync(L.dcount, 0, sizeof(int) * (size_t)c->n, c->stream));
-            k_defer_ranges<<<grid_for(nr, 256), 256, 0, c->stream>>>(kk, nr, (uint64_t)c->pcap, L.dstart, L.dcount);
+            k_defer_ranges<<<grid_for(nr, 256), 256, 0, c->stream>>>(kk, nr, (uint64_t)c->pcap, L.dstart, L.dcount,
+                                                                    c->d_status);
             mp.y = L.y;
             mp.skeys = kk;
             mp.svals = vv;

@@ -23,6 +23,6 @@ int exclusive_scan(const unsigned long long* in, unsigned long long* out, long l
 
 size_t radix_scratch_bytes(int n);
 int radix_sort(uint64_t*& keys, uint32_t*& vals, uint64_t*& keys_alt, uint32_t*& vals_alt, int n, int bits,
-                void* scratch, cudaStream_t st);
+                void* scratch, int* gave_up, cudaStream_t st);
 
 }  // namespace sphgpu

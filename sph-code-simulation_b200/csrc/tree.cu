@@ -81,24 +81,48 @@ __global__ void k_bbox_partial(const double4* __restrict__ pos, int n, double* _
 
 // Root cube of BHTree::make (src/bhtree.cpp:67-103) or BHTree::initialize
 // (src/bhtree.cpp:19-32) for periodic runs.
-__global__ void k_root(const double* __restrict__ part, int nparts, DevParams P, double4* __restrict__ root)
+// One block reduces the partial boxes (one thread took 288 us for the 1,024
+// of a million particles).
+__global__ void __launch_bounds__(BLK) k_root(const double* __restrict__ part, int nparts, DevParams P,
+                                              double4* __restrict__ root)
 {
-    if(threadIdx.x != 0) return;
+    __shared__ double s_box[BLK / 32][6];
     double lo[3], hi[3];
     if(P.periodic) {
         for(int k = 0; k < 3; ++k) {
             lo[k] = P.lo[k];
             hi[k] = P.hi[k];
         }
+        if(threadIdx.x != 0) return;
     } else {
         for(int k = 0; k < 3; ++k) {
             lo[k] = DBL_MAX;
             hi[k] = -DBL_MAX;
         }
-        for(int b = 0; b < nparts; ++b) {
+        for(int b = threadIdx.x; b < nparts; b += BLK) {
             for(int k = 0; k < 3; ++k) {
                 lo[k] = fmin(lo[k], part[b * 6 + k]);
                 hi[k] = fmax(hi[k], part[b * 6 + 3 + k]);
+            }
+        }
+        for(int o = 16; o > 0; o >>= 1) {
+            for(int k = 0; k < 3; ++k) {
+                lo[k] = fmin(lo[k], __shfl_xor_sync(FULL_MASK, lo[k], o));
+                hi[k] = fmax(hi[k], __shfl_xor_sync(FULL_MASK, hi[k], o));
+            }
+        }
+        if((threadIdx.x & 31) == 0) {
+            for(int k = 0; k < 3; ++k) {
+                s_box[threadIdx.x >> 5][k] = lo[k];
+                s_box[threadIdx.x >> 5][3 + k] = hi[k];
+            }
+        }
+        __syncthreads();
+        if(threadIdx.x != 0) return;
+        for(int w = 1; w < BLK / 32; ++w) {
+            for(int k = 0; k < 3; ++k) {
+                lo[k] = fmin(lo[k], s_box[w][k]);
+                hi[k] = fmax(hi[k], s_box[w][3 + k]);
             }
         }
         // BHTree::make under more than one OpenMP thread: the min / max
@@ -230,6 +254,7 @@ __global__ void k_nodes(const uint64_t* __restrict__ keys, int n, int D, const i
 {
     const int p = blockIdx.x * blockDim.x + threadIdx.x;
     if(p >= n) return;
+    if(st->pass_guard & PASS_GUARD_SORT) return;  // the keys are not sorted: the host reports it
     const double4 r = *root;
     if(p == 0) {
         const int total = base[n - 1] + nstart[n - 1] + 1;
@@ -416,13 +441,24 @@ __global__ void k_mass_up(int n, const int* __restrict__ leaf_of_start, DevTree 
         const int done = atomicAdd(&T.counter[par], 1);
         if(done != T.nchild[par] - 1) return;
         __threadfence();
-        const int stop = T.link[par].z;
+        // children in index order (the child table: their loads do not wait
+        // on one another as along the skip links)
         double m = 0.0, cx = 0.0, cy = 0.0, cz = 0.0;
-        int nch = 0;
-        for(int ch = par + 1; ch != stop && nch < 8; ch = T.link[ch].z, ++nch) {
-            const double2* q2 = reinterpret_cast<const double2*>(&T.mass[ch]);
+        const int4* kids = reinterpret_cast<const int4*>(T.child + (size_t)par * 8);
+        const int4 ka = kids[0], kb = kids[1];
+        const int kid[8] = {ka.x, ka.y, ka.z, ka.w, kb.x, kb.y, kb.z, kb.w};
+        double4 rec[8];
+#pragma unroll
+        for(int k = 0; k < 8; ++k) {
+            if(kid[k] < 0) continue;
+            const double2* q2 = reinterpret_cast<const double2*>(&T.mass[kid[k]]);
             const double2 lo = __ldcg(q2), hi = __ldcg(q2 + 1);
-            const double4 mc = make_double4(lo.x, lo.y, hi.x, hi.y);
+            rec[k] = make_double4(lo.x, lo.y, hi.x, hi.y);
+        }
+#pragma unroll
+        for(int k = 0; k < 8; ++k) {
+            if(kid[k] < 0) continue;
+            const double4 mc = rec[k];
             m = __dadd_rn(m, mc.w);
             cx = __dadd_rn(cx, __dmul_rn(mc.x, mc.w));
             cy = __dadd_rn(cy, __dmul_rn(mc.y, mc.w));
@@ -466,13 +502,15 @@ __global__ void k_ksize_up(int n, const int* __restrict__ leaf_of_start, DevTree
         const int done = atomicAdd(&T.counter[par], 1);
         if(done != T.nchild[par] - 1) return;
         __threadfence();
-        const int stop = T.link[par].z;
         double k = 0.0;
-        int nch = 0;
-        for(int ch = par + 1; ch != stop && nch < 8; ch = T.link[ch].z, ++nch) {
-            const double h = __ldcg(&T.ksize[ch]);
-            if(h > k) k = h;
-        }
+        const int4* kids = reinterpret_cast<const int4*>(T.child + (size_t)par * 8);
+        const int4 ka = kids[0], kb = kids[1];
+        const int kid[8] = {ka.x, ka.y, ka.z, ka.w, kb.x, kb.y, kb.z, kb.w};
+        double h[8];
+#pragma unroll
+        for(int q = 0; q < 8; ++q) h[q] = kid[q] >= 0 ? __ldcg(&T.ksize[kid[q]]) : 0.0;
+#pragma unroll
+        for(int q = 0; q < 8; ++q) k = h[q] > k ? h[q] : k;
         T.ksize[par] = k;
         node = par;
     }
@@ -499,10 +537,11 @@ int tree_make(sphgpu_ctx* c)
     SPHGPU_CUDA(c, cudaMemsetAsync(&c->d_status->node_pool, 0, 3 * sizeof(int), st));
     k_bbox_partial<<<nb, BLK, 0, st>>>(c->s.pos, n, c->d_bbox_part, c->d_status);
     ++launches;
-    k_root<<<1, 32, 0, st>>>(c->d_bbox_part, nb, c->dp, c->d_root);
+    k_root<<<1, BLK, 0, st>>>(c->d_bbox_part, nb, c->dp, c->d_root);
     // keys + sort
     k_keys<<<grid_for(n, BLK), BLK, 0, st>>>(c->s.pos, n, c->d_root, D, c->d_keys, c->d_vals);
-    launches += radix_sort(c->d_keys, c->d_vals, c->d_keys_alt, c->d_vals_alt, n, 3 * D, c->d_radix_scratch, st);
+    launches += radix_sort(c->d_keys, c->d_vals, c->d_keys_alt, c->d_vals_alt, n, 3 * D, c->d_radix_scratch,
+                           &c->d_status->pass_guard, st);
     // nodes
     k_levels<<<grid_for(n, BLK), BLK, 0, st>>>(c->d_keys, n, D, c->prm.leaf_particle_num, c->d_nstart, c->d_lvl);
     launches += exclusive_scan(c->d_nstart, c->d_base, n, (int*)nullptr, c->scan, st);

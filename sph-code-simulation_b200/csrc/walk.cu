@@ -836,7 +836,8 @@ __global__ void k_skin_check(DevParams P, DevState S, int n, const double* __res
 {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if(i >= n) return;
-    if(!(skin_need_radius(P, S, i, xb, *dmax, delta) < fr[i])) *bad = 1;
+    // (one store is enough: two million of them to one word took 0.25 ms)
+    if(!(skin_need_radius(P, S, i, xb, *dmax, delta) < fr[i]) && *reinterpret_cast<volatile int*>(bad) == 0) *bad = 1;
 }
 
 // After a failed check: the largest skin any particle needed, in units of the
