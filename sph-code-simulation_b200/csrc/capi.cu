@@ -229,7 +229,7 @@ int alloc_all(sphgpu_ctx* c, int n)
     if((rc = dalloc(c, c->d_root, 1)) || (rc = dalloc(c, c->d_bbox_part, 6 * 1024)) || (rc = dalloc(c, c->d_keys, n))
        || (rc = dalloc(c, c->d_keys_alt, n)) || (rc = dalloc(c, c->d_vals, n)) || (rc = dalloc(c, c->d_vals_alt, n))
        || (rc = dalloc(c, c->d_nstart, n)) || (rc = dalloc(c, c->d_base, n)) || (rc = dalloc(c, c->d_lvl, n))
-       || (rc = dalloc(c, c->d_leaf_of_start, n)) || (rc = dalloc(c, c->d_inv, n)) || (rc = dalloc(c, c->d_gcount, n))
+       || (rc = dalloc(c, c->d_leaf_of_start, n)) || (rc = dalloc(c, c->d_inv, n)) || (rc = dalloc(c, c->d_gcount, n)) || (rc = dalloc(c, c->d_split, (n / 32 + 1) * 5 / 4 + 2))
        || (rc = dalloc(c, c->d_pcount, n)) || (rc = dalloc(c, c->d_dt, 1)) || (rc = dalloc(c, c->d_hvs, 1))
        || (rc = dalloc(c, c->d_red, 8 + 6 * 1024 + 64)) || (rc = dalloc(c, c->d_status, 1)))
         return rc;

@@ -87,6 +87,7 @@ struct DevStatus {
     int overflow;          // a neighbour list exceeded the current capacity
     int fatal;             // a list exceeded neighbor_number * 1000
     int max_count;         // largest list seen
+    int split_windows;     // windows of the group walk that go by sub-groups
     int node_pool;         // node pool exhausted
     int guard;             // a neighbour walk hit its node-count bound (corrupt tree)
     int nonfinite;         // a particle position is NaN or infinite
@@ -430,6 +431,48 @@ struct KernH {
         const T a = T(0.5) * (T(2) - q + fabs(T(2) - q));
         const T b = T(0.5) * (T(1) - q + fabs(T(1) - q));
         return dhn * (a * a * (T(1.5) * q - T(1.5)) + b * b * (T(-6) * q + T(3)));
+    }
+};
+
+// The same kernels for the pair sums, without their h-dependent factors (the
+// sums are multiplied by wn, dwn, dhn of KernH once): W = wn w, grad W = r_ij
+// dwn dw, dW/dh = dhn dh, at q = r KernH::inv.  `in`: the pair counts; outside
+// the shape is zero, so masked pairs add zeros.  Inside, the reference's
+// (x + |x|) / 2 of 1 - q (2 - q) is that difference itself.
+template <typename T, int KER>
+struct Shape {
+    T q, a, b;  // Wendland: a = 1 - q; cubic: a = 2 - q, b = (1 - q)+; Gaussian: a = exp(-q^2)
+    __device__ __forceinline__ Shape(T q_, bool in) : q(q_)
+    {
+        if constexpr(KER == SPHGPU_GAUSSIAN) {
+            a = in ? exp(-(q * q)) : T(0);
+            b = T(0);
+        } else if constexpr(KER == SPHGPU_WENDLAND) {
+            a = in ? T(1) - q : T(0);
+            const T a2 = a * a;
+            b = a2 * a2 * a;
+        } else {
+            a = in ? T(2) - q : T(0);
+            b = in && q < T(1) ? T(1) - q : T(0);
+        }
+    }
+    __device__ __forceinline__ T w() const
+    {
+        if constexpr(KER == SPHGPU_GAUSSIAN) return a;
+        else if constexpr(KER == SPHGPU_WENDLAND) return (b * a) * (T(1) + q * (T(6) + q * T(35.0 / 3.0)));
+        else return T(0.25) * a * a * a - b * b * b;
+    }
+    __device__ __forceinline__ T dw(T rinv) const
+    {
+        if constexpr(KER == SPHGPU_GAUSSIAN) return a * q * rinv;
+        else if constexpr(KER == SPHGPU_WENDLAND) return b * (T(1) + T(5) * q);
+        else return rinv * (T(0.75) * a * a - T(3) * b * b);
+    }
+    __device__ __forceinline__ T dh() const
+    {
+        if constexpr(KER == SPHGPU_GAUSSIAN) return a * (T(2) * (q * q) - T(3));
+        else if constexpr(KER == SPHGPU_WENDLAND) return b * (T(9) + q * (T(45) + q * (T(-5) + q * T(-385))));
+        else return a * a * (T(1.5) * q - T(1.5)) + b * b * (T(-6) * q + T(3));
     }
 };
 

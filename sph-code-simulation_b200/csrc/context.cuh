@@ -46,6 +46,7 @@ struct sphgpu_ctx {
     // neighbour lists (ELL: capacity slots per particle, row-major)
     int* d_glist = nullptr;          // gather list (PreInteraction)
     int* d_gcount = nullptr;
+    int* d_split = nullptr;          // windows the group walk takes by sub-groups, then every window's width (bytes)
     int64_t gcap = 0;
     int* d_plist = nullptr;          // symmetric list (FluidForce)
     int* d_pcount = nullptr;

@@ -212,16 +212,6 @@ __device__ __forceinline__ double interval_gap(double c, double lo, double hi)
     return c < lo ? lo - c : (c > hi ? c - hi : 0.0);
 }
 
-// Periodic axis of length L, a group of extent ext, a candidate at offset b
-// (minimum image) from its centre.  A lane at offset a, |a| <= ext / 2, may
-// take d = a - b for the pair's offset when |d| <= L / 2 for sure; and else
-// when every image is further than h: then |d| > L / 2 > h, and the nearest
-// image is at least L / 2 - ext / 2 away.
-__device__ __forceinline__ bool image_safe(double b, double ext, double L, double h)
-{
-    return fabs(b) + 0.5 * ext < 0.499999 * L || 0.499999 * L - 0.5 * ext > h * (1.0 + 1e-6);
-}
-
 // exact box test of the reference's recursion at node nd for particle i
 template <bool IJ>
 __device__ __forceinline__ bool box_pass(const DevParams& P, const DevTree& T, int nd, double xi, double yi, double zi,
@@ -242,33 +232,31 @@ __device__ __forceinline__ bool box_pass(const DevParams& P, const DevTree& T, i
     return m <= l2;
 }
 
-// RES: resident blocks per SM (caps the registers).  9 (112 registers) where
-// the launch fills the chip: 1 M shear 2.98 -> 2.82 ms, 2 M tube 3.42 -> 3.22;
-// 8 (128 registers) where a warp's own latency counts: 137 K sphere 0.93 ->
-// 0.81, 17 K 0.215 -> 0.185.  The line is about four rounds of blocks.
+// RES: resident blocks per SM (caps the registers).  10 (96 registers) where
+// the launch fills the chip: 1 M shear 3.14 -> 2.97 ms, 2 M tube 3.69 -> 3.48; 8
+// (128 registers) where a warp's own latency counts: 137 K sphere 0.99 -> 0.87,
+// 17 K 0.232 -> 0.205.  The line is about four rounds of blocks.
 constexpr int GW_FEW = 148 * 8 * GW_WARPS * 32 * 4;
-template <bool IJ, int RES>
-__global__ void __launch_bounds__(GW_WARPS * 32, RES) k_walk_group(DevParams P, DevState S, DevTree T, int n, int cap,
-                                                             int* __restrict__ list, int* __restrict__ count,
-                                                             DevStatus* __restrict__ st, int guess, double ratio,
-                                                             SkinOut sk)
+// The walk's windows of 32 octree-ordered particles, a warp each: the search
+// radii (gather walk: the h guess), and the sub-groups.  A window that straddles
+// a large octant boundary has a bounding box far wider than its particles'
+// search spheres.  Such a window is walked in aligned sub-groups of s lanes (s =
+// 16, ..., 1: the largest s for which every sub-group's extent is at most
+// GW_SPLIT times its largest radius), each by a warp of its own; the others
+// whole.  (One warp for all of a window's sub-groups, up to 32 walks, was the
+// walk's tail: 17 K sphere 0.385 ms against 0.19.)
+constexpr int GW_WBLK = 256;
+__global__ void __launch_bounds__(GW_WBLK) k_walk_windows(DevParams P, DevState S, int n, int guess, double ratio,
+                                                         SkinOut sk, DevStatus* __restrict__ st,
+                                                         unsigned char* __restrict__ width, int* __restrict__ split)
 {
-    __shared__ int s_stack[GW_WARPS][GW_STACK];
-    __shared__ int s_queue[GW_WARPS][GW_QUEUE];
-    __shared__ __align__(16) float s_cx[GW_WARPS][32], s_cy[GW_WARPS][32], s_cz[GW_WARPS][32];
-    __shared__ double4 s_cpos[GW_WARPS][32];
-    __shared__ __align__(16) int s_cid[GW_WARPS][32];
-    __shared__ float2 s_ct[GW_WARPS][IJ ? 32 : 1];
-    const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int i = (blockIdx.x * GW_WARPS + w) * 32 + lane;
+    const int i = blockIdx.x * GW_WBLK + threadIdx.x, lane = threadIdx.x & 31;
     const bool valid = i < n;
     if(__ballot_sync(FULL_MASK, valid) == 0) return;  // whole warp past the end
-    double xi = 0, yi = 0, zi = 0, hi = 0;
+    double4 p = make_double4(0, 0, 0, 0);
+    double hi = 0;
     if(valid) {
-        const double4 p = S.pos[i];
-        xi = p.x;
-        yi = p.y;
-        zi = p.z;
+        p = S.pos[i];
         if(guess) {
             constexpr double A = 4.0 * 3.14159265358979323846 / 3.0;
             const double g = pow(P.nngb * p.w / (S.thermo[i].x * A), 1.0 / 3) * ratio;
@@ -282,63 +270,82 @@ __global__ void __launch_bounds__(GW_WARPS * 32, RES) k_walk_group(DevParams P, 
             hi = S.vel[i].w;
         }
     }
+    double lo[3] = {valid ? p.x : 1e300, valid ? p.y : 1e300, valid ? p.z : 1e300};
+    double up[3] = {valid ? p.x : -1e300, valid ? p.y : -1e300, valid ? p.z : -1e300};
+    double hm = valid ? hi : 0.0;
+    int s = 1;
+    for(int o = 1; o < 32; o <<= 1) {
+        for(int k = 0; k < 3; ++k) {
+            lo[k] = fmin(lo[k], __shfl_xor_sync(FULL_MASK, lo[k], o));
+            up[k] = fmax(up[k], __shfl_xor_sync(FULL_MASK, up[k], o));
+        }
+        hm = fmax(hm, __shfl_xor_sync(FULL_MASK, hm, o));
+        const double e = fmax(up[0] - lo[0], fmax(up[1] - lo[1], up[2] - lo[2]));
+        if(__all_sync(FULL_MASK, e <= GW_SPLIT * hm)) s = 2 * o;
+    }
+    if(lane == 0) {
+        width[i >> 5] = (unsigned char)s;
+        atomicAdd(s == 32 ? &st->walk_group_warps : &st->walk_split_warps, 1ull);
+        if(s < 32) split[atomicAdd(&st->split_windows, 1)] = i >> 5;
+    }
+}
+
+// The first `nsplit` blocks take the sub-groups of the split windows (32 items
+// per window, of which 32 / s are some), a warp each, beside the others, which
+// take a whole window per warp.
+template <bool IJ, int RES>
+__global__ void __launch_bounds__(GW_WARPS * 32, RES) k_walk_group(DevParams P, DevState S, DevTree T, int n, int cap,
+                                                             int* __restrict__ list, int* __restrict__ count,
+                                                             DevStatus* __restrict__ st, double factor, int nsplit,
+                                                             const unsigned char* __restrict__ width,
+                                                             const int* __restrict__ split)
+{
+    __shared__ int s_stack[GW_WARPS][GW_STACK];
+    __shared__ int s_queue[GW_WARPS][GW_QUEUE];
+    __shared__ __align__(16) float s_cx[GW_WARPS][32], s_cy[GW_WARPS][32], s_cz[GW_WARPS][32];
+    __shared__ double4 s_cpos[GW_WARPS][32];
+    __shared__ __align__(16) int s_cid[GW_WARPS][32];
+    __shared__ float2 s_ct[GW_WARPS][IJ ? 32 : 1];
+    const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
     // safety margin for the fast acceptance (see above)
     const double4 root = ldg4(&T.geo[0]);
     const double scale = fmax(fabs(root.x), fmax(fabs(root.y), fabs(root.z))) + root.w;
     const double delta = 1e-12 * scale;
-
-    int* out = list + (size_t)(valid ? i : 0) * (size_t)cap;
-    int cnt = 0;
-    int4 four = make_int4(0, 0, 0, 0);  // the last entries taken
-    bool overflow = false;
-    // Sub-groups.  A window of 32 octree-ordered particles that straddles a
-    // large octant boundary has a bounding box far wider than its particles'
-    // search spheres.  The warp takes runs of lanes whose extent is at most
-    // GW_SPLIT times their largest radius, from the first lane on, each run up
-    // to the jump that breaks it, and walks once per run: all lanes traverse
-    // and stage, the run's lanes test candidates.  (Halving the window until
-    // every aligned part fits put all 32 lanes of a window whose jump lies at
-    // an odd lane into walks of their own, the kernel's tail: 17 K sphere 0.385
-    // -> 0.245 ms, 2 M tube 4.94 -> 3.86.)
-    int first = 0;
-    while(first < 32 && !overflow) {
-        const bool in = valid && lane >= first;
-        double blo[3] = {in ? xi : 1e300, in ? yi : 1e300, in ? zi : 1e300};
-        double bup[3] = {in ? xi : -1e300, in ? yi : -1e300, in ? zi : -1e300};
-        double bh = in ? hi : 0.0;
-        for(int o = 1; o < 32; o <<= 1) {
-            // the box of lanes first .. this one
-            const bool take = lane - o >= first;
-            for(int k = 0; k < 3; ++k) {
-                const double l = __shfl_up_sync(FULL_MASK, blo[k], o), u = __shfl_up_sync(FULL_MASK, bup[k], o);
-                if(take) {
-                    blo[k] = fmin(blo[k], l);
-                    bup[k] = fmax(bup[k], u);
-                }
-            }
-            const double m = __shfl_up_sync(FULL_MASK, bh, o);
-            if(take) bh = fmax(bh, m);
+    const bool parts = (int)blockIdx.x < nsplit;
+    const int items = parts ? 32 * st->split_windows : (n + 31) / 32;
+    const int step = parts ? nsplit * GW_WARPS : items;
+    for(int item = (parts ? blockIdx.x : blockIdx.x - nsplit) * GW_WARPS + w; item < items; item += step) {
+        const int window = parts ? split[item >> 5] : item;
+        const int s = width[window], sg = parts ? item & 31 : 0;
+        if(parts ? sg >= 32 / s : s < 32) continue;
+        const int i = window * 32 + lane;
+        const bool valid = i < n;
+        double xi = 0, yi = 0, zi = 0, hi = 0;
+        if(valid) {
+            const double4 p = S.pos[i];
+            xi = p.x;
+            yi = p.y;
+            zi = p.z;
+            hi = S.vel[i].w * factor;
         }
-        bool fits = true;
-        for(int k = 0; k < 3; ++k) {
-            const double ext = bup[k] - blo[k];
-            fits = fits && ext <= GW_SPLIT * bh;
-            // a periodic axis: extents for which image_safe holds everywhere,
-            // unless the box is too short for any
-            const double most = P.range[k] - 2.02 * bh;
-            if(P.periodic && most > 0.0) fits = fits && ext < most;
-        }
-        const unsigned far = __ballot_sync(FULL_MASK, in && lane > first && !fits);
-        const int last = far ? __ffs(far) - 2 : 31;
-        for(int k = 0; k < 3; ++k) {
-            blo[k] = __shfl_sync(FULL_MASK, blo[k], last);
-            bup[k] = __shfl_sync(FULL_MASK, bup[k], last);
-        }
-        bh = __shfl_sync(FULL_MASK, bh, last);
-        const bool act = in && lane <= last;
-        if(lane == 0 && first == 0) atomicAdd(far ? &st->walk_split_warps : &st->walk_group_warps, 1ull);
-        first = last + 1;
+        // all lanes traverse and stage, the (sub-)group's lanes test candidates
+        const bool act = valid && lane / s == sg;
         if(__ballot_sync(FULL_MASK, act) == 0) continue;
+        double blo[3] = {act ? xi : 1e300, act ? yi : 1e300, act ? zi : 1e300};
+        double bup[3] = {act ? xi : -1e300, act ? yi : -1e300, act ? zi : -1e300};
+        double bh = act ? hi : 0.0;
+        for(int o = 1; o < 32; o <<= 1) {
+            for(int k = 0; k < 3; ++k) {
+                blo[k] = fmin(blo[k], __shfl_xor_sync(FULL_MASK, blo[k], o));
+                bup[k] = fmax(bup[k], __shfl_xor_sync(FULL_MASK, bup[k], o));
+            }
+            bh = fmax(bh, __shfl_xor_sync(FULL_MASK, bh, o));
+        }
+
+        int* out = list + (size_t)(valid ? i : 0) * (size_t)cap;
+        int cnt = 0;
+        int4 four = make_int4(0, 0, 0, 0);  // the last entries taken
+        bool overflow = false;
         const double bext = fmax(bup[0] - blo[0], fmax(bup[1] - blo[1], bup[2] - blo[2]));
         int sp = 0, nq = 0;
         if(lane == 0) s_stack[w][0] = 0;
@@ -357,31 +364,39 @@ __global__ void __launch_bounds__(GW_WARPS * 32, RES) k_walk_group(DevParams P, 
         // both thresholds rounded outwards to FP32.  A pair below Tin is in the
         // reference's set with every box test on its path passing (see above),
         // so it is taken without FP64 work; only pairs between the thresholds run
-        // the exact FP64 test.  With periodic wrapping the FP32 offset is the
-        // minimum image only if |b_j| + ext/2 < L/2 on every axis (|a_i| <= ext/2);
-        // and where it is not, the pair is certainly outside either way if
-        // image_safe holds; other candidates always run the exact test (most of
-        // a thin periodic box's did without image_safe's second case: 131 K shear
-        // layer 1.31 -> 0.63 ms, 245 K tube 1.44 -> 0.69).
+        // the exact FP64 test.  With periodic wrapping the FP32 offset may be
+        // another than the minimum image for some lane (|a_i| <= ext/2).  Where
+        // L/2 - ext/2 > h on every axis the pair is then outside either way
+        // (|d| > L/2 > h, and its nearest image is L/2 - ext/2 away or more) and
+        // nothing need be done.  Otherwise (`wide`: a thin box) each lane takes
+        // the nearest image in FP32, which costs E another 2^-22 L.  (Candidates
+        // that might have another image used to run the exact test for every
+        // lane: 131 K shear layer 1.31 ms, 245 K tube 1.44 ms, now 0.64 and 0.61.)
         // Each lane classifies a chunk of 32 staged candidates branch-free into
         // two bit masks (inside, band), runs the exact test for the band bits and
         // writes the taken candidates in chunk order.  Issue-bound (1 M shear: 60 K
         // instructions a warp for 59 chunks, 61 % of the issue slots): two
         // candidates per packed FP32 operation, each mask bit one funnel shift of a
         // sign, the candidates' nodes found by ballots, the next chunk's positions
-        // in flight (3.33 -> 2.82 ms; scalar FP32 3.01).
+        // in flight (1 M shear 3.33 -> 2.82 ms when it came; scalar FP32 3.01).
         const double cx = 0.5 * (blo[0] + bup[0]), cy = 0.5 * (blo[1] + bup[1]), cz = 0.5 * (blo[2] + bup[2]);
         const double ext_x = bup[0] - blo[0], ext_y = bup[1] - blo[1], ext_z = bup[2] - blo[2];
         const float ax = (float)(xi - cx), ay = (float)(yi - cy), az = (float)(zi - cz);
+        bool wide = false;
+        if(P.periodic) {
+            wide = IJ || ext_x > P.range[0] - 2.02 * bh || ext_y > P.range[1] - 2.02 * bh
+                || ext_z > P.range[2] - 2.02 * bh;
+        }
+        const double image_err = wide ? 0x1p-21 * fmax(P.range[0], fmax(P.range[1], P.range[2])) : 0.0;
         auto t_out = [&](double h) -> float {
-            const double t = h * (1.0 + 0x1p-20) + 0x1p-21 * bext;
+            const double t = h * (1.0 + 0x1p-20) + 0x1p-21 * bext + image_err;
             return __double2float_ru(t * t * (1.0 + 0x1p-20));
         };
         auto t_in = [&](double h) -> float {
-            const double t = (h - delta - (0x1p-22 * bext + 0x1p-21 * h)) * (1.0 - 0x1p-20);
+            const double t = (h - delta - (0x1p-22 * bext + 0x1p-21 * h + image_err)) * (1.0 - 0x1p-20);
             // (a radius below about 2^-20 of the extent: band pairs only, so that
             // Tout < 2 t^2 wherever a pair may be taken without the exact test)
-            const double o = h * (1.0 + 0x1p-20) + 0x1p-21 * bext;
+            const double o = h * (1.0 + 0x1p-20) + 0x1p-21 * bext + image_err;
             return t > 0.0 && o * o < 1.9 * (t * t) ? __double2float_rd(t * t * (1.0 - 0x1p-20)) : -1.0f;
         };
         const float Ti_out = act ? t_out(hi) : -1.0f;
@@ -395,7 +410,7 @@ __global__ void __launch_bounds__(GW_WARPS * 32, RES) k_walk_group(DevParams P, 
         const float gap = Ti_out - Ti_in;
         const f32x2 G2 = pack2(gap, gap);
         const float F_INF = __int_as_float(0x7f800000);
-        const float F_NAN = __int_as_float(0x7fffffff);
+        const float Lx = (float)P.range[0], Ly = (float)P.range[1], Lz = (float)P.range[2];
 
         auto process = [&](int nproc) {
             // expand the queued nodes into their particles (warp prefix sum)
@@ -427,7 +442,6 @@ __global__ void __launch_bounds__(GW_WARPS * 32, RES) k_walk_group(DevParams P, 
                 const bool have = base + lane < total;
                 const int q = qn;
                 const double4 pj = pn;
-                bool pre = true;
                 float fx = F_INF, fy = F_INF, fz = F_INF;  // padding: infinitely far, never taken
                 float tko = -1.0f, tki = -1.0f;
                 if(have) {
@@ -437,11 +451,6 @@ __global__ void __launch_bounds__(GW_WARPS * 32, RES) k_walk_group(DevParams P, 
                         bx = min_image(bx, P.range[0]);
                         by = min_image(by, P.range[1]);
                         bz = min_image(bz, P.range[2]);
-                        // the offset is the minimum image for every lane, or the
-                        // axis alone keeps the pair apart either way round
-                        const double hk = IJ ? fmax(bh, ks) : bh;
-                        pre = image_safe(bx, ext_x, P.range[0], hk) && image_safe(by, ext_y, P.range[1], hk)
-                            && image_safe(bz, ext_z, P.range[2], hk);
                     }
                     if(IJ) {
                         tko = t_out(ks);
@@ -453,8 +462,6 @@ __global__ void __launch_bounds__(GW_WARPS * 32, RES) k_walk_group(DevParams P, 
                     s_cpos[w][lane] = make_double4(pj.x, pj.y, pj.z, ks);
                     s_cid[w][lane] = q;
                 }
-                // candidates whose image depends on the lane: exact tests
-                const unsigned force = __ballot_sync(FULL_MASK, !pre);
                 s_cx[w][lane] = -fx;
                 s_cy[w][lane] = -fy;
                 s_cz[w][lane] = -fz;
@@ -467,7 +474,7 @@ __global__ void __launch_bounds__(GW_WARPS * 32, RES) k_walk_group(DevParams P, 
                 unsigned in_mask = 0u;
                 if(act) {
                     unsigned band_mask = 0u;
-                    if constexpr(!IJ) {
+                    if(!IJ && !wide) {
                         unsigned near = 0u, inside = 0u;
 #pragma unroll
                         for(int k = 28; k >= 0; k -= 4) {
@@ -488,13 +495,18 @@ __global__ void __launch_bounds__(GW_WARPS * 32, RES) k_walk_group(DevParams P, 
                             inside = sign_in(inside, hi32(ta));
                             inside = sign_in(inside, lo32(ta));
                         }
-                        in_mask = inside & ~force;
-                        band_mask = (near & ~inside) | force;
+                        in_mask = inside;
+                        band_mask = near & ~inside;
                     } else {
 #pragma unroll
                         for(int k = 0; k < 32; ++k) {
-                            const float dx = ax + s_cx[w][k], dy = ay + s_cy[w][k], dz = az + s_cz[w][k];
-                            const float2 tk = s_ct[w][k];
+                            float dx = ax + s_cx[w][k], dy = ay + s_cy[w][k], dz = az + s_cz[w][k];
+                            if(wide) {
+                                dx = fabsf(dx) > 0.5f * Lx ? dx - copysignf(Lx, dx) : dx;
+                                dy = fabsf(dy) > 0.5f * Ly ? dy - copysignf(Ly, dy) : dy;
+                                dz = fabsf(dz) > 0.5f * Lz ? dz - copysignf(Lz, dz) : dz;
+                            }
+                            const float2 tk = IJ ? s_ct[w][k] : make_float2(-1.0f, -1.0f);
                             const float r2f = fmaf(dz, dz, fmaf(dy, dy, dx * dx));
                             const float to = fmaxf(Ti_out, tk.x);
                             const float ti = fmaxf(Ti_in, tk.y);
@@ -503,8 +515,6 @@ __global__ void __launch_bounds__(GW_WARPS * 32, RES) k_walk_group(DevParams P, 
                             in_mask |= (unsigned)inside << k;
                             band_mask |= (unsigned)band << k;
                         }
-                        in_mask &= ~force;
-                        band_mask |= force;
                     }
                     while(band_mask) {
                         const int k = __ffs(band_mask) - 1;
@@ -631,25 +641,26 @@ __global__ void __launch_bounds__(GW_WARPS * 32, RES) k_walk_group(DevParams P, 
             }
         }
         if(!overflow && nq > 0) process(nq);
-    }
-    if(overflow) {
-        if(lane == 0) st->guard = 2;
-        return;
-    }
-    if(valid) {
-        // the entries past the last whole four
-        const int rem = cnt & 3;
-        if(cnt <= cap) {
-            if(rem == 3) out[cnt - 3] = four.y;
-            if(rem >= 2) out[cnt - 2] = four.z;
-            if(rem >= 1) out[cnt - 1] = four.w;
+        if(overflow) {
+            if(lane == 0) st->guard = 2;
+            return;
         }
-        count[i] = cnt;
-        if(cnt > cap) st->overflow = 1;
-        if(cnt > P.nngb * 1000) st->fatal = 1;
+        if(act) {
+            // the entries past the last whole four
+            const int rem = cnt & 3;
+            if(cnt <= cap) {
+                if(rem == 3) out[cnt - 3] = four.y;
+                if(rem >= 2) out[cnt - 2] = four.z;
+                if(rem >= 1) out[cnt - 1] = four.w;
+            }
+            count[i] = cnt;
+            if(cnt > cap) st->overflow = 1;
+            if(cnt > P.nngb * 1000) st->fatal = 1;
+        }
+        const int longest = __reduce_max_sync(FULL_MASK, act ? cnt : 0);
+        if(lane == 0) atomicMax(&st->max_count, longest);
+        __syncwarp();
     }
-    const int longest = __reduce_max_sync(FULL_MASK, valid ? cnt : 0);
-    if(lane == 0) atomicMax(&st->max_count, longest);
 }
 
 // exhaustive_search (src/exhaustive_search.cpp:11-42): all j with
@@ -713,22 +724,25 @@ int run_walk(sphgpu_ctx* c, int which, bool guess, double ratio, bool exhaustive
         const int64_t cap = which == 0 ? c->gcap : c->pcap;
         int* list = which == 0 ? c->d_glist : c->d_plist;
         int* count = which == 0 ? c->d_gcount : c->d_pcount;
-        SPHGPU_CUDA(c, cudaMemsetAsync(c->d_status, 0, 3 * sizeof(int), st));
+        static_assert(offsetof(DevStatus, split_windows) == 3 * sizeof(int), "status word layout");
+        SPHGPU_CUDA(c, cudaMemsetAsync(c->d_status, 0, 4 * sizeof(int), st));
         SPHGPU_CUDA(c, cudaMemsetAsync(&c->d_status->guard, 0, sizeof(int), st));
         if(exhaustive) {
             k_exhaustive<<<grid_for(n, 128), 128, 0, st>>>(c->dp, c->s, n, is_ij, (int)cap, list, count, c->d_status);
         } else if(c->walk_mode == 0 && !per_lane) {
             const unsigned grid = grid_for(n, GW_WARPS * 32);
             const bool few = n <= GW_FEW;
-            if(which == 0) {
-                auto* k = few ? k_walk_group<false, 8> : k_walk_group<false, 9>;
-                k<<<grid, GW_WARPS * 32, 0, st>>>(c->dp, c->s, c->t, n, (int)cap, list, count, c->d_status,
-                                                  guess ? 1 : 0, ratio, sk);
-            } else {
-                auto* k = few ? k_walk_group<true, 8> : k_walk_group<true, 9>;
-                k<<<grid, GW_WARPS * 32, 0, st>>>(c->dp, c->s, c->t, n, (int)cap, list, count, c->d_status, 0, 1.0,
-                                                  SkinOut{1.0, nullptr, nullptr});
-            }
+            const int nsplit = (int)std::min<long long>(16LL * grid, 148 * 2);
+            unsigned char* width = reinterpret_cast<unsigned char*>(c->d_split + (n / 32 + 1));
+            k_walk_windows<<<grid_for(n, GW_WBLK), GW_WBLK, 0, st>>>(c->dp, c->s, n, which == 0 && guess ? 1 : 0, ratio,
+                                                                     which == 0 ? sk : SkinOut{1.0, nullptr, nullptr},
+                                                                     c->d_status, width, c->d_split);
+            auto* k = which == 0 ? (few ? k_walk_group<false, 8> : k_walk_group<false, 10>)
+                                 : (few ? k_walk_group<true, 8> : k_walk_group<true, 10>);
+            k<<<nsplit + grid, GW_WARPS * 32, 0, st>>>(c->dp, c->s, c->t, n, (int)cap, list, count, c->d_status,
+                                                       which == 0 && guess ? sk.factor : 1.0, nsplit, width,
+                                                       c->d_split);
+            ++*launches;
         } else if(which == 0) {
             k_walk<false><<<grid_for(n, WBLK), WBLK, 0, st>>>(c->dp, c->s, c->t, n, (int)cap, list, count,
                                                             c->d_status, guess ? 1 : 0, ratio, sk);
@@ -737,10 +751,10 @@ int run_walk(sphgpu_ctx* c, int which, bool guess, double ratio, bool exhaustive
                                                            c->d_status, 0, 1.0, SkinOut{1.0, nullptr, nullptr});
         }
         SPHGPU_LAUNCH_CHECK(c, "neighbour walk");
-        // the first seven status words: the walk's own and the pass guard of
+        // the first eight status words: the walk's own and the pass guard of
         // the bottom-up mass pass that ran before it
-        static_assert(offsetof(DevStatus, pass_guard) == 6 * sizeof(int), "status word layout");
-        SPHGPU_CUDA(c, cudaMemcpyAsync(&c->h_status, c->d_status, 7 * sizeof(int), cudaMemcpyDeviceToHost, st));
+        static_assert(offsetof(DevStatus, pass_guard) == 7 * sizeof(int), "status word layout");
+        SPHGPU_CUDA(c, cudaMemcpyAsync(&c->h_status, c->d_status, 8 * sizeof(int), cudaMemcpyDeviceToHost, st));
         SPHGPU_CUDA(c, cudaStreamSynchronize(st));
         if(c->h_status.fatal) {
             return fail(c, SPHGPU_ERR_NEIGHBOR_OVERFLOW,
