@@ -12,14 +12,16 @@
 // r >= max(h_i, h_j) or r == 0 exactly as the reference; acc and du/dt are
 // accumulated in FP64 and group-reduced, then overwrite acc (the reference
 // overwrites too; gravity adds afterwards).
-// T = double: plain FP64 form.  T = float: pair arithmetic in FP32 with FP64
-// accumulators (mixed form); the Riemann Newton iteration runs in FP32 and its
-// final step in FP64.
+// k_force64: plain FP64 form.  k_force_mixed: pair arithmetic in FP32 with FP64
+// accumulators; the Riemann Newton iteration runs in FP32 and its final step in
+// FP64.
 #include <cfloat>
+#include <type_traits>
 #include <cuda_runtime.h>
 
 #include "context.cuh"
 #include "mlp.cuh"
+#include "rounded.cuh"
 #include "scan_sort.cuh"
 
 namespace sphgpu {
@@ -27,6 +29,12 @@ namespace sphgpu {
 namespace {
 
 constexpr int FBLK = 256;
+// FP64 form: threads per block and resident blocks per SM (which cap the
+// registers).  ssph, disph: 128 registers without spills (3 blocks: disph 1.82
+// -> 2.26 ms on the 1.1 M sphere).  gsph, gdisph: 168 registers, 12 warps
+// (2 M gsph tube 6.67 -> 6.36 ms against 16 warps that spill).
+constexpr int force64_threads(int type) { return type == SPHGPU_GSPH || type == SPHGPU_GDISPH ? 64 : 256; }
+constexpr int force64_blocks(int type) { return type == SPHGPU_GSPH || type == SPHGPU_GDISPH ? 6 : 2; }
 
 template <typename T>
 struct V3 {
@@ -208,18 +216,6 @@ __device__ void riemann_iterative(const double* L, const double* R, double gamma
 // learned guess, deferring the pairs whose linearised start the screen
 // rejects (their features and pair slots go to the MlpPairs rows); 4 = the
 // deferred pairs only, with the network's guess, added to acc.
-// Minimum resident blocks per SM (caps registers; measured on B200): FP64
-// disph 2 (27.2 -> 24.5 ms on the 8.78 M sphere), FP64 gdisph 3 (8.8 -> 7.7 ms
-// on the 2 M tube), FP32 disph 3 (17.3 -> 16.0 ms, once the next pair's index
-// is fetched ahead), gsph and the other FP32 forms 4 (gsph 18.8 -> 9.6 ms
-// against 3), FP64 ssph 3.
-template <typename T, int TYPE>
-constexpr int force_min_blocks()
-{
-    if(sizeof(T) == sizeof(float) && TYPE == SPHGPU_DISPH) return 3;
-    if(sizeof(T) == sizeof(float) || TYPE == SPHGPU_GSPH) return 4;
-    return TYPE == SPHGPU_DISPH ? 2 : 3;
-}
 
 // The particles a launch computes: all n, or (sub.idx != null) the listed
 // ones (the mixed form's FP64 re-evaluation).  count = 0: the launch adds to
@@ -230,14 +226,16 @@ struct Subset {
     int count;
 };
 
-template <typename T, int G, int TYPE, int MODE>
-__global__ void __launch_bounds__(FBLK, (force_min_blocks<T, TYPE>())) k_force(DevParams P, DevState S, int n, const int* __restrict__ list,
+// The mixed form: pair arithmetic in FP32, accumulators in FP64.  Resident
+// blocks per SM measured: disph 3 (17.3 -> 16.0 ms on the 8.8 M sphere), others 4.
+template <int G, int TYPE, int MODE>
+__global__ void __launch_bounds__(FBLK, (TYPE == SPHGPU_DISPH ? 3 : 4)) k_force_mixed(DevParams P, DevState S, int n, const int* __restrict__ list,
                                                 const int* __restrict__ count, int cap, const double* __restrict__ dtp,
                                                 DevStatus* __restrict__ st, MlpPairs mp, Harvest hv,
                                                 float* __restrict__ accabs, Subset sub)
 {
+    using T = float;
     constexpr int GPW = 32 / G;
-    constexpr bool f32 = sizeof(T) == sizeof(float);
     const int lane = threadIdx.x & (G - 1);
     const long long warp = ((long long)blockIdx.x * FBLK + threadIdx.x) >> 5;
     const long long nwarps = ((long long)gridDim.x * FBLK) >> 5;
@@ -298,20 +296,14 @@ __global__ void __launch_bounds__(FBLK, (force_min_blocks<T, TYPE>())) k_force(D
             const double4 vj = ldg4(&S.vel[j]);
             const double hj = vj.w;
             double r, rinv;
-            if constexpr(f32) {
-                // the set predicate in FP64 (exact), the distance in FP32
-                const double r2 = abs2x(d);
-                if(!root_lt(r2, hi < hj ? hj : hi) || r2 == 0.0) continue;
-                const float r2f = (float)r2;
-                const float rif = rsqrtf(r2f);
-                r = (double)(r2f * rif);
-                rinv = (double)rif;
-                if(!(r > 0.0)) continue;  // r^2 below FP32's range: coincident for the force
-            } else {
-                r = sqrt(abs2x(d));
-                if(r >= (hi < hj ? hj : hi) || r == 0.0) continue;
-                rinv = 1.0 / r;
-            }
+            // the set predicate in FP64 (exact), the distance in FP32
+            const double r2 = abs2x(d);
+            if(!root_lt(r2, hi < hj ? hj : hi) || r2 == 0.0) continue;
+            const float r2f = (float)r2;
+            const float rif = rsqrtf(r2f);
+            r = (double)(r2f * rif);
+            rinv = (double)rif;
+            if(!(r > 0.0)) continue;  // r^2 below FP32's range: coincident for the force
             ++n_pairs;
             const double4 tj = ldg4(&S.thermo[j]);
             const T rT = (T)r;
@@ -375,16 +367,11 @@ __global__ void __launch_bounds__(FBLK, (force_min_blocks<T, TYPE>())) k_force(D
                     Lst[3] = tj.w;
                 }
                 if(TYPE == SPHGPU_GDISPH) {
-                    double pg, vg;
-                    if(sizeof(T) == sizeof(double)) {
-                        riemann_hll<double>(Lst, Rst, pg, vg);
-                    } else {
-                        const float Lf[4] = {(float)Lst[0], (float)Lst[1], (float)Lst[2], (float)Lst[3]};
-                        const float Rf[4] = {(float)Rst[0], (float)Rst[1], (float)Rst[2], (float)Rst[3]};
-                        float ps, vs;
-                        riemann_hll<float>(Lf, Rf, ps, vs);
-                        pg = ps;
-                    }
+                    const float Lf[4] = {(float)Lst[0], (float)Lst[1], (float)Lst[2], (float)Lst[3]};
+                    const float Rf[4] = {(float)Rst[0], (float)Rst[1], (float)Rst[2], (float)Rst[3]};
+                    float ps, vs;
+                    riemann_hll<float>(Lf, Rf, ps, vs);
+                    const double pg = ps;
                     psi = (T)pg / Pi;
                     psj = (T)pg / Pj;
                 }
@@ -439,8 +426,6 @@ __global__ void __launch_bounds__(FBLK, (force_min_blocks<T, TYPE>())) k_force(D
                                 }
                             }
                         }
-                    } else if(sizeof(T) == sizeof(double)) {
-                        riemann_hll<double>(Lst, Rst, pstar, vstar);
                     } else {
                         const float Lf[4] = {(float)Lst[0], (float)Lst[1], (float)Lst[2], (float)Lst[3]};
                         const float Rf[4] = {(float)Rst[0], (float)Rst[1], (float)Rst[2], (float)Rst[3]};
@@ -459,7 +444,7 @@ __global__ void __launch_bounds__(FBLK, (force_min_blocks<T, TYPE>())) k_force(D
                     ax -= fx;
                     ay -= fy;
                     az -= fz;
-                    if constexpr(f32) sabs += (float)(fabs(fx) + fabs(fy) + fabs(fz));
+                    sabs += (float)(fabs(fx) + fabs(fy) + fabs(fz));
                     de -= fx * (ex * vstar - vi.x) + fy * (ey * vstar - vi.y) + fz * (ez * vstar - vi.z);
                     continue;
                 }
@@ -503,22 +488,22 @@ __global__ void __launch_bounds__(FBLK, (force_min_blocks<T, TYPE>())) k_force(D
             ay -= (double)fy;
             az -= (double)fz;
             de += (double)e_;
-            if constexpr(f32) sabs += fabsf(fx) + fabsf(fy) + fabsf(fz);
+            sabs += fabsf(fx) + fabsf(fy) + fabsf(fz);
         }
         ax = group_sum<G>(ax);
         ay = group_sum<G>(ay);
         az = group_sum<G>(az);
         de = group_sum<G>(de);
-        if constexpr(f32) sabs = group_sum<G>(sabs);
+        sabs = group_sum<G>(sabs);
         if(MODE == 4) {
             if(cnt > 0 && lane == 0) {
                 const double4 a0 = S.acc[i];
                 S.acc[i] = make_double4(a0.x + ax, a0.y + ay, a0.z + az, a0.w + de);
-                if(f32 && accabs) accabs[i] += sabs;
+                if(accabs) accabs[i] += sabs;
             }
         } else if(valid && lane == 0) {
             S.acc[i] = make_double4(ax, ay, az, de);
-            if(f32 && accabs) accabs[i] = sabs;
+            if(accabs) accabs[i] = sabs;
         }
     }
     if(!sub.count) return;
@@ -540,38 +525,453 @@ __global__ void __launch_bounds__(FBLK, (force_min_blocks<T, TYPE>())) k_force(D
     }
 }
 
-constexpr int GROUP = 4;
-
-unsigned force_grid(int n)
+// ---------------------------------------------------------------- FP64 form
+// d W / dr factor of one smoothing length without its pair terms: grad W =
+// r_ij dwn Shape::dw
+template <int KER>
+__device__ __forceinline__ double dwn_of(double inv)
 {
-    const long long gpb = FBLK / GROUP;
-    const long long blocks = (n + gpb - 1) / gpb;
-    return (unsigned)std::max<long long>(1, std::min<long long>(blocks, 148LL * 8 * 4));
+    constexpr double PI = 3.14159265358979323846;
+    if constexpr(KER == SPHGPU_GAUSSIAN) return -2.0 * (GAUSS_SIGMA * inv * inv * inv) * inv;
+    else if constexpr(KER == SPHGPU_WENDLAND) return -56.0 / 3.0 * (495.0 / (32.0 * PI)) * (inv * inv * inv) * inv * inv;
+    else return -(1.0 / PI) * (inv * inv * inv) * inv;
+}
+// KernH::inv: 1 / h, of the cubic spline 2 / h
+template <int KER>
+constexpr double kern_span() { return KER == SPHGPU_CUBIC_SPLINE ? 2.0 : 1.0; }
+
+// van Leer limiter (limiter above) without a branch
+template <typename Op>
+__device__ __forceinline__ double limit(Op& op, double dq1, double dq2)
+{
+    const double p = dq1 * dq2;
+    const bool some = p > 0.0;
+    const double q = op.div(some ? 2.0 * p : 1.0, some ? dq1 + dq2 : 1.0);
+    return p <= 0.0 ? 0.0 : q;
 }
 
-template <typename T, int MODE>
-void launch_force(sphgpu_ctx* c, MlpPairs mp, Harvest hv, Subset sub = {nullptr, 0, 1})
+// riemann_hll with the pair's operations
+template <typename Op>
+__device__ __forceinline__ void hll(Op& op, const double* L, const double* R, double& pstar, double& vstar)
 {
-    const unsigned grid = force_grid(sub.idx ? sub.n : c->n);
-    const int type = c->prm.sph_type;
-    float* accabs = sizeof(T) == sizeof(float) ? c->d_accabs : nullptr;
-    if(type == SPHGPU_DISPH) {
-        k_force<T, GROUP, SPHGPU_DISPH, 0><<<grid, FBLK, 0, c->stream>>>(c->dp, c->s, c->n, c->d_plist, c->d_pcount,
-                                                                         (int)c->pcap, c->d_dt, c->d_status, mp, hv,
-                                                                         accabs, sub);
-    } else if(type == SPHGPU_GSPH) {
-        k_force<T, GROUP, SPHGPU_GSPH, MODE><<<grid, FBLK, 0, c->stream>>>(c->dp, c->s, c->n, c->d_plist,
-                                                                           c->d_pcount, (int)c->pcap, c->d_dt,
-                                                                           c->d_status, mp, hv, accabs, sub);
-    } else if(type == SPHGPU_GDISPH) {
-        k_force<T, GROUP, SPHGPU_GDISPH, 0><<<grid, FBLK, 0, c->stream>>>(c->dp, c->s, c->n, c->d_plist,
-                                                                          c->d_pcount, (int)c->pcap, c->d_dt,
-                                                                          c->d_status, mp, hv, accabs, sub);
-    } else {
-        k_force<T, GROUP, SPHGPU_SSPH, 0><<<grid, FBLK, 0, c->stream>>>(c->dp, c->s, c->n, c->d_plist, c->d_pcount,
-                                                                        (int)c->pcap, c->d_dt, c->d_status, mp, hv,
-                                                                        accabs, sub);
+    const double rl = op.root(L[1]), rr = op.root(R[1]);
+    const double inv = op.inverse(rl + rr);
+    const double ut = (rl * L[0] + rr * R[0]) * inv;
+    const double ct = (rl * L[3] + rr * R[3]) * inv;
+    const double sl = fmin(L[0] - L[3], ut - ct);
+    const double sr = fmax(R[0] + R[3], ut + ct);
+    const double c1 = L[1] * (sl - L[0]);
+    const double c2 = R[1] * (sr - R[0]);
+    const double c3 = op.inverse(c1 - c2);
+    const double c4 = L[2] - L[0] * c1;
+    const double c5 = R[2] - R[0] * c2;
+    vstar = (c5 - c4) * c3;
+    pstar = (c1 * c5 - c2 * c4) * c3;
+}
+
+// riemann_iterative<double> from the linearised start, with the pair's
+// operations; the quotients by p_L and p_R share their reciprocals.
+template <typename Op>
+__device__ __forceinline__ void iterate_star(Op& op, const double* L, const double* R, double gamma, double tol,
+                                             double& pstar, double& vstar, int& iters)
+{
+    const double ul = L[0], pl = L[2], ur = R[0], pr = R[2];
+    iters = 0;
+    if(L[1] < 0.0 || R[1] < 0.0 || pl < 0.0 || pr < 0.0) {
+        pstar = 0.0;
+        vstar = 0.0;
+        return;
     }
+    const double g2 = 1.0 + gamma;
+    const double g1 = 0.5 * g2 / gamma;
+    const double vl = op.inverse(L[1]), vr = op.inverse(R[1]);
+    const double cl = op.root(gamma * pl * L[1]), cr = op.root(gamma * pr * R[1]);
+    const double yl = op.inverse(pl), yr = op.inverse(pr);
+    double p = pr - pl - cr * (ur - ul);
+    p = pl + op.div0(p * cl, cl + cr);
+    p = fmax(p, 1e-25);
+    auto speed = [&](double q, double ps, double y, double c) {
+        return c * op.root(1.0 + op.over(g1 * (q - ps), ps, y));
+    };
+    for(int it = 0; it < 20; ++it) {
+        const double pold = p;
+        const double wl = speed(p, pl, yl, cl), wr = speed(p, pr, yr, cr);
+        double zl = 4.0 * vl * wl * wl;
+        zl = op.div(-zl * wl, zl - g2 * (p - pl));
+        double zr = 4.0 * vr * wr * wr;
+        zr = op.div(zr * wr, zr - g2 * (p - pr));
+        const double usl = ul - op.div0(p - pl, wl);
+        const double usr = ur + op.div0(p - pr, wr);
+        p = p + op.div0((usr - usl) * (zl * zr), zr - zl);
+        p = fmax(1e-25, p);
+        ++iters;
+        if(fabs(p - pold) < tol * p || (Op::quick && op.bad)) break;
+    }
+    pstar = p;
+    const double wl = speed(p, pl, yl, cl), wr = speed(p, pr, yr, cr);
+    const double usl = ul - op.div0(p - pl, wl);
+    const double usr = ur + op.div0(p - pr, wr);
+    vstar = 0.5 * (usl + usr);
+}
+
+// The FP64 form, with the kernel function and the periodic box at
+// compile time.  What bounds it: issue slots and the FP64 pipe at 16 warps per
+// SM, the pair's quotients and roots above all (disph five, gsph thirty: in the
+// general form each is a branch to a special-case path and a chain of its own;
+// here Quick, and a pair whose operands leave its range again with Ieee).
+// Measured (general operations, kernel function at run time -> now): 1.1 M disph
+// sphere 2.84 -> 1.82 ms (41 % of the issue slots before, FP64 pipe 45 %), 1 M
+// shear layer 3.07 -> 1.99, 0.49 M ssph sphere 0.60 -> 0.36, 17 K 0.042 -> 0.024,
+// 244 K gdisph tube 0.97 -> 0.68, 2 M gsph tube 8.4 -> 6.4 (FP64 pipe 50 %).
+template <int G, int TYPE, int KER, bool PER, int MODE>
+__global__ void __launch_bounds__(force64_threads(TYPE), force64_blocks(TYPE)) k_force64(DevParams P, DevState S, int n, const int* __restrict__ list,
+                                                const int* __restrict__ count, int cap, const double* __restrict__ dtp,
+                                                DevStatus* __restrict__ st, MlpPairs mp, Harvest hv, Subset sub)
+{
+    constexpr int GPW = 32 / G;
+    constexpr bool gsph = TYPE == SPHGPU_GSPH, gdisph = TYPE == SPHGPU_GDISPH;
+    constexpr bool disph = TYPE == SPHGPU_DISPH || gdisph;
+    const int lane = threadIdx.x & (G - 1);
+    const long long warp = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    const long long nwarps = ((long long)gridDim.x * blockDim.x) >> 5;
+    const double dt = *dtp;
+    const double gamma = P.gamma;
+    unsigned long long solves = 0, iters = 0, fallbacks = 0;
+    unsigned n_cand = 0, n_pairs = 0;  // work counters of this lane
+    const int nloop = sub.idx ? sub.n : n;
+
+    for(long long wb = warp * GPW; wb < nloop; wb += nwarps * GPW) {
+        const int slot = (int)(wb + ((threadIdx.x & 31) / G));
+        const bool valid = slot < nloop;
+        const int i = sub.idx ? (valid ? sub.idx[slot] : n) : slot;
+        const int cnt = valid ? (MODE == 4 ? mp.dcount[i] : min(count[i], cap)) : 0;
+        if(MODE == 4 && !__any_sync(FULL_MASK, cnt > 0)) continue;
+        const int* li = list + (size_t)(valid ? i : 0) * (size_t)cap;
+        const double4 pi = valid ? S.pos[i] : make_double4(0, 0, 0, 0);
+        const double4 vi = valid ? S.vel[i] : make_double4(0, 0, 0, 1);
+        const double4 ti = valid ? S.thermo[i] : make_double4(1, 1, 1, 1);
+        const double4 si = valid ? S.visc[i] : make_double4(0, 0, 1, 0);
+        const double hi = vi.w;
+        double4 gi0 = make_double4(0, 0, 0, 0), gi1 = gi0, gi2 = gi0, gi3 = gi0;
+        if((gsph || gdisph) && P.gsph2 && valid) {
+            gi0 = S.grad[i];
+            gi1 = S.grad[(size_t)n + i];
+            gi2 = S.grad[2 * (size_t)n + i];
+            gi3 = S.grad[3 * (size_t)n + i];
+        }
+        const double rhoi = ti.x, Pi = ti.y, ui = ti.z, ci = ti.w;
+        const double inv_i = kern_span<KER>() / hi, dwn_i = dwn_of<KER>(inv_i);
+        // per-particle factors of the pair terms
+        const double ppr = Pi / (rhoi * rhoi);                  // ssph P_i / rho_i^2
+        const double g2u = (gamma - 1.0) * (gamma - 1.0) * ui;  // disph (gamma-1)^2 u_i
+        const double g2up = g2u / Pi;
+        const double mu_inv = 1.0 / (pi.w * ui);
+        const double r2i = 1.0 / (rhoi * rhoi);
+        double ax = 0, ay = 0, az = 0, de = 0;
+        n_cand += lane < cnt ? (unsigned)((cnt - lane + G - 1) / G) : 0u;
+        // the next pair's index is fetched one iteration ahead, so the
+        // neighbour's loads do not wait on the list load
+        int jn = MODE != 4 && lane < cnt ? __ldg(&li[lane]) : 0;
+        for(int k = lane; k < cnt; k += G) {
+            float yq = 0.f;
+            int j;
+            if(MODE == 4) {
+                const int row = mp.dstart[i] + k;
+                const int kk = (int)(mp.skeys[row] - (uint64_t)i * (uint64_t)cap);
+                yq = mp.y[mp.svals[row]];
+                j = li[kk];
+            } else {
+                j = jn;
+                if(k + G < cnt) jn = __ldg(&li[k + G]);
+            }
+            const double4 pj = ldg4(&S.pos[j]);
+            const double4 vj = ldg4(&S.vel[j]);
+            const double4 tj = ldg4(&S.thermo[j]);
+            Vec3d d{xsub(pi.x, pj.x), xsub(pi.y, pj.y), xsub(pi.z, pj.z)};
+            if constexpr(PER) {
+                d.x = min_image(d.x, P.range[0]);
+                d.y = min_image(d.y, P.range[1]);
+                d.z = min_image(d.z, P.range[2]);
+            }
+            const double hj = vj.w;
+            const double r2 = abs2x(d);
+            // r < max(h_i, h_j) and r > 0, as the reference decides them
+            if(!root_lt(r2, hi < hj ? hj : hi) || r2 == 0.0) continue;
+            ++n_pairs;
+            double4 sj = make_double4(0, 0, 0, 0);
+            if(!gsph) sj = ldg4(&S.visc[j]);
+
+            // the pair's terms; false: nothing is added now (deferred)
+            double fx, fy, fz, e_;
+            int it = 0, fb = 0;
+            double Lst[4], Rst[4], pstar = 0.0;
+            auto pair = [&](auto& op) -> bool {
+                double r, rinv;
+                if constexpr(std::remove_reference_t<decltype(op)>::quick) {
+                    const double y = rsqrt_near(r2);
+                    r = op.check(root_rn(r2, y));
+                    rinv = op.check(recip_rn(r, y));
+                } else {
+                    r = sqrt(r2);
+                    rinv = 1.0 / r;
+                }
+                const double inv_j = kern_span<KER>() * op.inverse(hj);  // (exact: a power of two)
+                const double qi = r * inv_i, qj = r * inv_j;
+                // (the reference's kernels vanish beyond their own h)
+                const Shape<double, KER> shi(qi, KER == SPHGPU_GAUSSIAN || qi < kern_span<KER>());
+                const Shape<double, KER> shj(qj, KER == SPHGPU_GAUSSIAN || qj < kern_span<KER>());
+                const double ci_ = dwn_i * shi.dw(rinv), cj_ = dwn_of<KER>(inv_j) * shj.dw(rinv);
+                const double mj = pj.w;
+                const double rhoj = tj.x, Pj = tj.y, cj = tj.w;
+                // gdisph: the HLL star pressure of the MUSCL states scales the disph
+                // pressure terms below by p_star / P_i and p_star / P_j
+                // (src/gdisph/gd_fluid_force.cpp:95-178)
+                [[maybe_unused]] double psi = 1.0, psj = 1.0;
+                if constexpr(gsph || gdisph) {
+                    const double ex = d.x * rinv, ey = d.y * rinv, ez = d.z * rinv;
+                    const double vei = vi.x * ex + vi.y * ey + vi.z * ez;
+                    const double vej = vj.x * ex + vj.y * ey + vj.z * ez;
+                    const bool hllc = gdisph || P.riemann != SPHGPU_RIEMANN_ITERATIVE;
+                    if(P.gsph2) {
+                        // MUSCL reconstruction (src/gsph/g_fluid_force.cpp:103-140)
+                        const double4 gj0 = ldg4(&S.grad[j]), gj1 = ldg4(&S.grad[(size_t)n + j]);
+                        const double4 gj2 = ldg4(&S.grad[2 * (size_t)n + j]), gj3 = ldg4(&S.grad[3 * (size_t)n + j]);
+                        const double di = 0.5 * (1.0 - ci * dt * rinv);
+                        const double dj = 0.5 * (1.0 - cj * dt * rinv);
+                        // velocity: dv_i[k] = grad_v[k] . e, dve_i = dv_i . e * r
+                        const double dvi0 = gi1.z * ex + gi1.w * ey + gi2.x * ez;
+                        const double dvi1 = gi2.y * ex + gi2.z * ey + gi2.w * ez;
+                        const double dvi2 = gi3.x * ex + gi3.y * ey + gi3.z * ez;
+                        const double dvj0 = gj1.z * ex + gj1.w * ey + gj2.x * ez;
+                        const double dvj1 = gj2.y * ex + gj2.z * ey + gj2.w * ez;
+                        const double dvj2 = gj3.x * ex + gj3.y * ey + gj3.z * ez;
+                        const double dve_i = (dvi0 * ex + dvi1 * ey + dvi2 * ez) * r;
+                        const double dve_j = (dvj0 * ex + dvj1 * ey + dvj2 * ez) * r;
+                        const double dv_ij = vei - vej;
+                        Rst[0] = vei - limit(op, dv_ij, dve_i) * di;
+                        Lst[0] = vej + limit(op, dv_ij, dve_j) * dj;
+                        const double dd_ij = rhoi - rhoj;
+                        const double dd_i = (gi0.x * ex + gi0.y * ey + gi0.z * ez) * r;
+                        const double dd_j = (gj0.x * ex + gj0.y * ey + gj0.z * ez) * r;
+                        Rst[1] = rhoi - limit(op, dd_ij, dd_i) * di;
+                        Lst[1] = rhoj + limit(op, dd_ij, dd_j) * dj;
+                        const double dp_ij = Pi - Pj;
+                        const double dp_i = (gi0.w * ex + gi1.x * ey + gi1.y * ez) * r;
+                        const double dp_j = (gj0.w * ex + gj1.x * ey + gj1.y * ez) * r;
+                        Rst[2] = Pi - limit(op, dp_ij, dp_i) * di;
+                        Lst[2] = Pj + limit(op, dp_ij, dp_j) * dj;
+                        if(hllc) {
+                            Rst[3] = op.root(op.div(gamma * Rst[2], Rst[1]));
+                            Lst[3] = op.root(op.div(gamma * Lst[2], Lst[1]));
+                        }
+                    } else {
+                        Rst[0] = vei;
+                        Rst[1] = ti.x;
+                        Rst[2] = ti.y;
+                        Rst[3] = ti.w;
+                        Lst[0] = vej;
+                        Lst[1] = tj.x;
+                        Lst[2] = tj.y;
+                        Lst[3] = tj.w;
+                    }
+                    if constexpr(gdisph) {
+                        double pg, vg;
+                        hll(op, Lst, Rst, pg, vg);
+                        psi = pg / Pi;
+                        psj = op.div(pg, Pj);
+                    } else {
+                        double vstar;
+                        if constexpr(MODE == 3 || MODE == 4) {
+                            const bool states_ok = Lst[1] > 0.0 && Rst[1] > 0.0 && Lst[2] > 0.0 && Rst[2] > 0.0;
+                            double scr_ch = -1.0, scr_q1 = 0.0;
+                            if(MODE == 3 && states_ok) pair_screen(Lst, Rst, gamma, scr_ch, scr_q1);
+                            if(MODE == 3 && !(scr_ch < 1e-2) && states_ok) {
+                                // deferred to the completion pass, which solves it from
+                                // the network's guess; with the row list full the pair
+                                // is solved here from the linearised start instead
+                                if(op.bad) return false;  // (again with the general operations)
+                                const unsigned long long row = atomicAdd(mp.rows, 1ull);
+                                if((long long)row < mp.rcap) {
+                                    float x[MLP_IN];
+                                    mlp_features(Lst, Rst, gamma, x);
+                                    mp.feat[row] = make_uint4(pack_bf16x2(x[0], x[1]), pack_bf16x2(x[2], x[3]),
+                                                              pack_bf16x2(x[4], 0.f), 0u);
+                                    mp.keys[row] = (uint64_t)i * (uint64_t)cap + (uint64_t)k;
+                                    atomicAdd(&st->mlp_guesses, 1ull);
+                                    return false;
+                                }
+                            }
+                            // learned start: the linearised guess where the screen
+                            // accepts it, else the network's (a NaN guess selects
+                            // the linearised one)
+                            riemann_iterative<double>(Lst, Rst, gamma, states_ok, MODE == 4 ? yq : __int_as_float(0x7fc00000),
+                                                      P.mlp_max_newton, pstar, vstar, it, fb, scr_ch, scr_q1, P.riemann_tol);
+                        } else if(hllc) {
+                            hll(op, Lst, Rst, pstar, vstar);
+                        } else {
+                            iterate_star(op, Lst, Rst, gamma, P.riemann_tol, pstar, vstar, it);
+                        }
+                        // f = dw_i m_j p* / rho_i^2 + dw_j m_j p* / rho_j^2 (src/gsph/g_fluid_force.cpp:158-165)
+                        const double fi = mj * pstar * r2i * ci_;
+                        const double fj = mj * pstar * op.inverse(rhoj * rhoj) * cj_;
+                        fx = -(d.x * (fi + fj));
+                        fy = -(d.y * (fi + fj));
+                        fz = -(d.z * (fi + fj));
+                        e_ = fx * (ex * vstar - vi.x) + fy * (ey * vstar - vi.y) + fz * (ez * vstar - vi.z);
+                        return true;
+                    }
+                }
+                if constexpr(!gsph) {
+                    const double uj = tj.z;
+                    const double cij = (ci_ + cj_) * 0.5;
+                    const double vx = vi.x - vj.x, vy = vi.y - vj.y, vz = vi.z - vj.z;
+                    const double vr = vx * d.x + vy * d.y + vz * d.z;
+                    const double sum = rhoi + rhoj, ysum = op.inverse(sum);
+                    // artificial viscosity (src/fluid_force.cpp:88-106)
+                    const double w = vr * rinv;
+                    const double visc = -0.5 * (0.5 * (si.y + sj.y)) * (0.5 * (si.x + sj.x)) * (ci + cj - 3.0 * w) * w
+                        * op.over(2.0, sum, ysum);
+                    const double pij = vr < 0.0 ? visc : 0.0;
+                    // artificial conductivity (src/fluid_force.cpp:108-116)
+                    double dac = 0.0;
+                    if(P.use_ac) {
+                        const double vs = P.gravity ? fabs(w) : op.root0(op.over(2.0 * fabs(Pi - Pj), sum, ysum));
+                        dac = P.alpha_ac * mj * vs * (ui - uj) * (cij * r2) * rinv;
+                    }
+                    double a_i, a_j, t_;
+                    if constexpr(disph) {
+                        const double mu = mj * uj;
+                        const double fij = 1.0 - op.div0(si.z, mu);
+                        const double fji = 1.0 - sj.z * mu_inv;
+                        t_ = g2up * uj * fij * psi;
+                        a_i = mj * (t_ + 0.5 * pij);
+                        a_j = mj * (g2u * op.div(uj, Pj) * fji * psj + 0.5 * pij);
+                    } else {
+                        t_ = ppr * si.z;
+                        a_i = mj * (t_ + 0.5 * pij);
+                        a_j = mj * (op.div(Pj, rhoj * rhoj) * sj.z + 0.5 * pij);
+                    }
+                    e_ = mj * t_ * (vr * ci_) + 0.5 * mj * pij * (vr * cij) + dac;
+                    const double f = ci_ * a_i + cj_ * a_j;
+                    fx = -(d.x * f);
+                    fy = -(d.y * f);
+                    fz = -(d.z * f);
+                }
+                return true;
+            };
+            Quick quick;
+            bool done = pair(quick);
+            if(quick.bad) {
+                Ieee ieee;
+                done = pair(ieee);
+            }
+            if(!done) continue;
+            if constexpr(gsph) {
+                if(P.riemann == SPHGPU_RIEMANN_ITERATIVE) {
+                    ++solves;
+                    iters += it;
+                    fallbacks += fb;
+                    if(MODE == 0 && hv.mod) {
+                        unsigned hsh = (unsigned)i * 0x9E3779B1u ^ (unsigned)k * 0x85EBCA77u ^ hv.salt;
+                        hsh ^= hsh >> 15;
+                        hsh *= 0x2C1B3C6Du;
+                        hsh ^= hsh >> 12;
+                        if(hsh % hv.mod == 0) {
+                            const unsigned long long at = atomicAdd(hv.count, 1ull);
+                            if((long long)at < hv.cap) {
+                                double* o = hv.out + 8 * at;
+                                o[0] = Lst[0];
+                                o[1] = Lst[1];
+                                o[2] = Lst[2];
+                                o[3] = Rst[0];
+                                o[4] = Rst[1];
+                                o[5] = Rst[2];
+                                o[6] = gamma;
+                                o[7] = pstar;
+                            }
+                        }
+                    }
+                }
+            }
+            ax += fx;
+            ay += fy;
+            az += fz;
+            de += e_;
+        }
+        ax = group_sum<G>(ax);
+        ay = group_sum<G>(ay);
+        az = group_sum<G>(az);
+        de = group_sum<G>(de);
+        if(MODE == 4) {
+            if(cnt > 0 && lane == 0) {
+                const double4 a0 = S.acc[i];
+                S.acc[i] = make_double4(a0.x + ax, a0.y + ay, a0.z + az, a0.w + de);
+            }
+        } else if(valid && lane == 0) {
+            S.acc[i] = make_double4(ax, ay, az, de);
+        }
+    }
+    if(!sub.count) return;
+    if(MODE != 4) {  // the completion pass re-solves pairs the force pass counted
+        block_count(&st->force_cand, n_cand);
+        block_count(&st->force_pairs, n_pairs);
+    }
+    if(gsph) {
+        for(int o = 16; o > 0; o >>= 1) {
+            solves += __shfl_xor_sync(FULL_MASK, solves, o);
+            iters += __shfl_xor_sync(FULL_MASK, iters, o);
+            fallbacks += __shfl_xor_sync(FULL_MASK, fallbacks, o);
+        }
+        if((threadIdx.x & 31) == 0 && solves) {
+            atomicAdd(&st->riemann_solves, solves);
+            atomicAdd(&st->riemann_iters, iters);
+            if(fallbacks) atomicAdd(&st->riemann_fallbacks, fallbacks);
+        }
+    }
+}
+
+constexpr int GROUP = 4;
+
+unsigned force_grid(int n, int threads = FBLK)
+{
+    const long long gpb = threads / GROUP;
+    const long long blocks = (n + gpb - 1) / gpb;
+    return (unsigned)std::max<long long>(1, std::min<long long>(blocks, 148LL * 8 * 4 * (FBLK / threads)));
+}
+
+template <int TYPE, int MODE>
+void launch_force_mixed(sphgpu_ctx* c, MlpPairs mp, Harvest hv, Subset sub)
+{
+    k_force_mixed<GROUP, TYPE, MODE><<<force_grid(c->n), FBLK, 0, c->stream>>>(
+        c->dp, c->s, c->n, c->d_plist, c->d_pcount, (int)c->pcap, c->d_dt, c->d_status, mp, hv, c->d_accabs, sub);
+}
+
+template <int TYPE, int MODE, int KER>
+void launch_force_form(sphgpu_ctx* c, MlpPairs mp, Harvest hv, Subset sub)
+{
+    auto* k = c->prm.periodic ? k_force64<GROUP, TYPE, KER, true, MODE> : k_force64<GROUP, TYPE, KER, false, MODE>;
+    constexpr int threads = force64_threads(TYPE);
+    k<<<force_grid(sub.idx ? sub.n : c->n, threads), threads, 0, c->stream>>>(
+        c->dp, c->s, c->n, c->d_plist, c->d_pcount, (int)c->pcap, c->d_dt, c->d_status, mp, hv, sub);
+}
+
+template <int TYPE, int MODE>
+void launch_force_type(sphgpu_ctx* c, bool mixed, MlpPairs mp, Harvest hv, Subset sub)
+{
+    if(mixed) launch_force_mixed<TYPE, MODE>(c, mp, hv, sub);
+    else if(c->prm.kernel == SPHGPU_WENDLAND) launch_force_form<TYPE, MODE, SPHGPU_WENDLAND>(c, mp, hv, sub);
+    else if(c->prm.kernel == SPHGPU_GAUSSIAN) launch_force_form<TYPE, MODE, SPHGPU_GAUSSIAN>(c, mp, hv, sub);
+    else launch_force_form<TYPE, MODE, SPHGPU_CUBIC_SPLINE>(c, mp, hv, sub);
+}
+
+template <int MODE>
+void launch_force(sphgpu_ctx* c, bool mixed, MlpPairs mp, Harvest hv, Subset sub = {nullptr, 0, 1})
+{
+    const int type = c->prm.sph_type;
+    if(type == SPHGPU_GSPH) launch_force_type<SPHGPU_GSPH, MODE>(c, mixed, mp, hv, sub);
+    else if(type == SPHGPU_DISPH) launch_force_type<SPHGPU_DISPH, 0>(c, mixed, mp, hv, sub);
+    else if(type == SPHGPU_GDISPH) launch_force_type<SPHGPU_GDISPH, 0>(c, mixed, mp, hv, sub);
+    else launch_force_type<SPHGPU_SSPH, 0>(c, mixed, mp, hv, sub);
 }
 
 // Riemann problems in bulk (labels and evaluation of the learned guess).
@@ -675,7 +1075,7 @@ int fluid_force_subset64(sphgpu_ctx* c, const int* idx, int nsub)
 {
     Harvest hv{};
     MlpPairs mp{};
-    launch_force<double, 0>(c, mp, hv, Subset{idx, nsub, 0});
+    launch_force<0>(c, false, mp, hv, Subset{idx, nsub, 0});
     SPHGPU_LAUNCH_CHECK(c, "FluidForce (FP64 re-evaluation)");
     return SPHGPU_OK;
 }
@@ -696,6 +1096,7 @@ int fluid_force(sphgpu_ctx* c)
     stage_begin(c, SPHGPU_T_FORCE);
     Harvest hv{c->d_harvest, c->d_harvest_count, c->harvest_cap, c->harvest_mod, 0u};
     MlpPairs mp{};
+    const bool mixed = c->prm.precision == SPHGPU_MIXED;
     int launches = 1;
     if(learned) {
         const int64_t slots = (int64_t)c->n * c->pcap;
@@ -722,8 +1123,7 @@ int fluid_force(sphgpu_ctx* c)
         mp.rows = L.rows;
         mp.rcap = c->mlp_rcap;
         // pass 1: every pair the screen accepts; the others become rows
-        if(c->prm.precision == SPHGPU_MIXED) launch_force<float, 3>(c, mp, hv);
-        else launch_force<double, 3>(c, mp, hv);
+        launch_force<3>(c, mixed, mp, hv);
         SPHGPU_LAUNCH_CHECK(c, "FluidForce");
         unsigned long long rows = 0;
         SPHGPU_CUDA(c, cudaMemcpyAsync(&rows, L.rows, sizeof(rows), cudaMemcpyDeviceToHost, c->stream));
@@ -751,13 +1151,11 @@ int fluid_force(sphgpu_ctx* c)
             mp.dstart = L.dstart;
             mp.dcount = L.dcount;
             // pass 2: the deferred pairs from the network's guess, added to acc
-            if(c->prm.precision == SPHGPU_MIXED) launch_force<float, 4>(c, mp, hv);
-            else launch_force<double, 4>(c, mp, hv);
+            launch_force<4>(c, mixed, mp, hv);
             launches += 2;
         }
     } else {
-        if(c->prm.precision == SPHGPU_MIXED) launch_force<float, 0>(c, mp, hv);
-        else launch_force<double, 0>(c, mp, hv);
+        launch_force<0>(c, mixed, mp, hv);
     }
     SPHGPU_LAUNCH_CHECK(c, "FluidForce");
     stage_end(c, SPHGPU_T_FORCE, launches);

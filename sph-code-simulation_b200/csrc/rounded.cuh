@@ -70,4 +70,58 @@ __device__ __forceinline__ double quot_rn(double a, double b, double y)
     return __fma_rn(__fma_rn(-b, q, a), y, q);
 }
 
+// Quotients and roots of one pair: Quick takes the forms above and notes when a
+// result may have left the range where they hold (its pair is then computed
+// again with Ieee); no branch in between, so independent operations overlap.
+// A result in 2^-400 .. 2^400 is the rounded one: an operand outside the
+// exponent range yields zero, infinity or NaN, and a residual that lost bits to
+// underflow needs operands below 2^-900.
+struct Ieee {
+    static constexpr bool quick = false;
+    bool bad = false;
+    __device__ __forceinline__ double inverse(double b) { return 1.0 / b; }
+    __device__ __forceinline__ double over(double a, double b, double) { return a / b; }
+    __device__ __forceinline__ double div(double a, double b) { return a / b; }
+    __device__ __forceinline__ double div0(double a, double b) { return a / b; }
+    __device__ __forceinline__ double root(double a) { return sqrt(a); }
+    __device__ __forceinline__ double root0(double a) { return sqrt(a); }
+};
+struct Quick {
+    static constexpr bool quick = true;
+    bool bad = false;
+    __device__ __forceinline__ double check(double q)
+    {
+        const unsigned hi = (unsigned)__double2hiint(q) & 0x7fffffffu;
+        bad = bad || hi - ((1023u - 400u) << 20) >= (800u << 20);
+        return q;
+    }
+    // 1 / b to about an ulp, for over()
+    __device__ __forceinline__ double near(double b)
+    {
+        const double y = rcp_seed(b);
+        const double e = __fma_rn(-b, y, 1.0);
+        return __fma_rn(y, __fma_rn(e, e, e), y);
+    }
+    // 1 / b
+    __device__ __forceinline__ double inverse(double b) { return check(recip_rn(b)); }
+    // a / b with y = 1 / b taken before; a may be zero
+    __device__ __forceinline__ double over(double a, double b, double y)
+    {
+        const double q = quot_rn(a, b, y);
+        if(a != 0.0) check(q);
+        return q;
+    }
+    __device__ __forceinline__ double div(double a, double b) { return check(quot_rn(a, b, near(b))); }
+    // a / b, a may be zero
+    __device__ __forceinline__ double div0(double a, double b)
+    {
+        const double y = near(b);
+        check(y);
+        return over(a, b, y);
+    }
+    __device__ __forceinline__ double root(double a) { return check(root_rn(a, rsqrt_near(a))); }
+    // sqrt(a), a may be zero
+    __device__ __forceinline__ double root0(double a) { return a > 0.0 ? root(a) : (check(a == 0.0 ? 1.0 : 0.0), 0.0); }
+};
+
 }  // namespace sphgpu
