@@ -18,7 +18,7 @@ struct sphgpu_ctx;
 namespace sphgpu {
 
 constexpr int MLP_IN = 5;
-constexpr int MLP_INP = 16;   // input padded to one k-step of m16n8k16
+constexpr int MLP_INP = 16;   // row length of the first layer in the image
 constexpr int MLP_H = 64;
 // FP32 master parameter layout:
 //   W0 [64][5], b0 [64], W1 [64][64], b1 [64], W2 [64][64], b2 [64], w3 [64], b3 [1]
@@ -33,13 +33,11 @@ constexpr int OFF_W3 = OFF_B2 + MLP_H;
 constexpr int OFF_B3 = OFF_W3 + MLP_H;
 
 // Device image (one allocation): BF16 W0p [64][16], W1 [64][64], W2 [64][64],
-// W1^T, W2^T (backward), then FP32 w3 [64], b0, b1, b2 [64], b3.
+// then FP32 w3 [64], b0, b1, b2 [64], b3.
 constexpr int IMG_W0 = 0;
 constexpr int IMG_W1 = IMG_W0 + MLP_H * MLP_INP;
 constexpr int IMG_W2 = IMG_W1 + MLP_H * MLP_H;
-constexpr int IMG_W1T = IMG_W2 + MLP_H * MLP_H;
-constexpr int IMG_W2T = IMG_W1T + MLP_H * MLP_H;
-constexpr int IMG_BF16 = IMG_W2T + MLP_H * MLP_H;              // bf16 elements
+constexpr int IMG_BF16 = IMG_W2 + MLP_H * MLP_H;               // bf16 elements
 constexpr int IMG_F32_OFFSET = ((IMG_BF16 * 2 + 255) / 256) * 256; // bytes
 constexpr int IMGF_W3 = 0, IMGF_B0 = 64, IMGF_B1 = 128, IMGF_B2 = 192, IMGF_B3 = 256;
 constexpr int IMG_F32 = 260;
