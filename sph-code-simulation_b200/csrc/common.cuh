@@ -248,31 +248,6 @@ __device__ __forceinline__ bool root_lt(double r2, double h)
     return sqrt(r2) < h;
 }
 
-// Pair loops: true when sqrt(r2) < h (exactly as root_lt); then r and 1/r.
-// Outside the band they come from one reciprocal square root (CUDA's rsqrt,
-// within an ulp of 1/sqrt), inside it from the correctly rounded root; for
-// r2 = 0 both are 0.  The pair sums built from them agree with the
-// reference's to rounding, as before; only set membership must be exact.
-__device__ __forceinline__ bool pair_within(double r2, double h, double& r, double& rinv)
-{
-    const double h2 = h * h;
-    if(r2 > h2 * (1.0 + 0x1p-40)) return false;
-    if(r2 >= h2 * (1.0 - 0x1p-40)) {
-        r = sqrt(r2);
-        if(!(r < h)) return false;
-        rinv = r > 0.0 ? 1.0 / r : 0.0;
-        return true;
-    }
-    if(r2 > 0.0) {
-        rinv = rsqrt(r2);
-        r = r2 * rinv;
-    } else {
-        r = 0.0;
-        rinv = 0.0;
-    }
-    return true;
-}
-
 // ------------------------------------------------------------ SPH kernels
 // W, grad W (as the scalar c with grad W = r_ij c) and dW/dh for the cubic
 // spline (include/kernel/cubic_spline.hpp:21-53), Wendland C4
@@ -431,6 +406,52 @@ struct KernH {
         const T a = T(0.5) * (T(2) - q + fabs(T(2) - q));
         const T b = T(0.5) * (T(1) - q + fabs(T(1) - q));
         return dhn * (a * a * (T(1.5) * q - T(1.5)) + b * b * (T(-6) * q + T(3)));
+    }
+};
+
+// KernH<float> with the kernel function at compile time, operation for operation:
+// the products that the switch on `type` keeps from being fused into what uses
+// them are rounded here too, so the mixed form's bits are the same.
+template <int KER>
+struct KernF {
+    KernH<float> k;
+    __device__ __forceinline__ explicit KernF(float h) : k(KER, h) {}
+    __device__ __forceinline__ float w(float r) const
+    {
+        const float q = __fmul_rn(r, k.inv);
+        if(KER == SPHGPU_GAUSSIAN) return __fmul_rn(k.wn, expf(-__fmul_rn(q, q)));
+        if(KER == SPHGPU_WENDLAND) {
+            const float a = 0.5f * (1.f - q + fabsf(1.f - q));
+            const float a2 = a * a;
+            return __fmul_rn(k.wn * (a2 * a2 * a2), 1.f + 6.f * q + float(35.0 / 3.0) * q * q);
+        }
+        const float a = 0.5f * (2.f - q + fabsf(2.f - q));
+        const float b = 0.5f * (1.f - q + fabsf(1.f - q));
+        return __fmul_rn(k.wn, 0.25f * a * a * a - b * b * b);
+    }
+    __device__ __forceinline__ float dwc(float r, float rinv) const
+    {
+        const float q = __fmul_rn(r, k.inv);
+        if(KER == SPHGPU_GAUSSIAN) return r == 0.f ? 0.f : __fmul_rn(k.dwn * expf(-__fmul_rn(q, q)) * q, rinv);
+        if(KER == SPHGPU_WENDLAND) return k.dwc(r, rinv);
+        const float a = 0.5f * (2.f - q + fabsf(2.f - q));
+        const float b = 0.5f * (1.f - q + fabsf(1.f - q));
+        return r == 0.f ? 0.f : __fmul_rn(k.dwn * rinv, 0.75f * a * a - 3.f * b * b);
+    }
+    __device__ __forceinline__ float dhw(float r) const
+    {
+        const float q = __fmul_rn(r, k.inv);
+        if(KER == SPHGPU_GAUSSIAN) {
+            return __fmul_rn(k.dhn * expf(-__fmul_rn(q, q)), 2.f * __fmul_rn(q, q) - 3.f);
+        }
+        if(KER == SPHGPU_WENDLAND) {
+            const float a = 0.5f * (1.f - q + fabsf(1.f - q));
+            const float a2 = a * a;
+            return __fmul_rn(k.dhn * (a2 * a2 * a), 9.f + 45.f * q + -5.f * q * q - 385.f * q * q * q);
+        }
+        const float a = 0.5f * (2.f - q + fabsf(2.f - q));
+        const float b = 0.5f * (1.f - q + fabsf(1.f - q));
+        return __fmul_rn(k.dhn, a * a * (1.5f * q - 1.5f) + b * b * (-6.f * q + 3.f));
     }
 };
 

@@ -35,6 +35,10 @@ constexpr int FBLK = 256;
 // (2 M gsph tube 6.67 -> 6.36 ms against 16 warps that spill).
 constexpr int force64_threads(int type) { return type == SPHGPU_GSPH || type == SPHGPU_GDISPH ? 64 : 256; }
 constexpr int force64_blocks(int type) { return type == SPHGPU_GSPH || type == SPHGPU_GDISPH ? 6 : 2; }
+// Resident blocks of the mixed form, measured: gsph 4 (2: 3.74 -> 4.13 ms on the
+// 1 M tube), gdisph 2 (4: 2.22 -> 2.54), ssph 3 (4: 0.349 -> 0.391, 2: 0.415),
+// disph 3 (2: 1.76 -> 2.01).
+constexpr int force_mixed_blocks(int type) { return type == SPHGPU_GSPH ? 4 : (type == SPHGPU_GDISPH ? 2 : 3); }
 
 template <typename T>
 struct V3 {
@@ -228,8 +232,21 @@ struct Subset {
 
 // The mixed form: pair arithmetic in FP32, accumulators in FP64.  Resident
 // blocks per SM measured: disph 3 (17.3 -> 16.0 ms on the 8.8 M sphere), others 4.
-template <int G, int TYPE, int MODE>
-__global__ void __launch_bounds__(FBLK, (TYPE == SPHGPU_DISPH ? 3 : 4)) k_force_mixed(DevParams P, DevState S, int n, const int* __restrict__ list,
+// The mixed form: pair arithmetic in FP32, distances, predicates and sums in
+// FP64.  Bound by the neighbour loads' latency and the conversions between the
+// two precisions (28 % of the pair loop's issue slots lost to loads in flight,
+// the conversions' unit 45 % busy).  The records of the predicate and of the pair
+// are loaded together (before, thermo waited for the predicate), the periodic box
+// and, for disph, the kernel function are compile-time, and the resident blocks
+// follow the registers: 1.1 M disph sphere 2.06 -> 1.76 ms, 131 K shear layer
+// 0.308 -> 0.258, 493 K ssph sphere 0.399 -> 0.351, 1 M gdisph tube 2.52 -> 2.25,
+// 125 K blast (both passes of the learned start) 2.51 -> 2.17.  The other forms
+// keep the kernel function a run-time switch read inside the loop: compile-time
+// (or hoisted, where the compiler splits the loop by it) it rounds their pair
+// terms differently, as products get fused into sums, for 2 %.
+constexpr int ANY_KERNEL = -1;
+template <int G, int TYPE, int KER, bool PER, int MODE>
+__global__ void __launch_bounds__(FBLK, force_mixed_blocks(TYPE)) k_force_mixed(DevParams P, DevState S, int n, const int* __restrict__ list,
                                                 const int* __restrict__ count, int cap, const double* __restrict__ dtp,
                                                 DevStatus* __restrict__ st, MlpPairs mp, Harvest hv,
                                                 float* __restrict__ accabs, Subset sub)
@@ -266,7 +283,7 @@ __global__ void __launch_bounds__(FBLK, (TYPE == SPHGPU_DISPH ? 3 : 4)) k_force_
         }
         const T rhoi = (T)ti.x, Pi = (T)ti.y, ui = (T)ti.z, ci = (T)ti.w;
         const T mi = (T)pi.w;
-        const KernH<T> khi(P.kernel, (T)hi);
+        const KernH<T> khi(KER == ANY_KERNEL ? P.kernel : KER, (T)hi);
         // per-particle factors of the pair terms
         const T ppr = Pi / (rhoi * rhoi);                             // ssph P_i / rho_i^2
         const T g2u = ((T)gamma - T(1)) * ((T)gamma - T(1)) * ui;     // disph (gamma-1)^2 u_i
@@ -292,8 +309,14 @@ __global__ void __launch_bounds__(FBLK, (TYPE == SPHGPU_DISPH ? 3 : 4)) k_force_
                 if(k + G < cnt) jn = __ldg(&li[k + G]);
             }
             const double4 pj = ldg4(&S.pos[j]);
-            const Vec3d d = rij(P, pi.x, pi.y, pi.z, pj.x, pj.y, pj.z);
             const double4 vj = ldg4(&S.vel[j]);
+            const double4 tj = ldg4(&S.thermo[j]);
+            Vec3d d{xsub(pi.x, pj.x), xsub(pi.y, pj.y), xsub(pi.z, pj.z)};
+            if constexpr(PER) {
+                d.x = min_image(d.x, P.range[0]);
+                d.y = min_image(d.y, P.range[1]);
+                d.z = min_image(d.z, P.range[2]);
+            }
             const double hj = vj.w;
             double r, rinv;
             // the set predicate in FP64 (exact), the distance in FP32
@@ -305,11 +328,12 @@ __global__ void __launch_bounds__(FBLK, (TYPE == SPHGPU_DISPH ? 3 : 4)) k_force_
             rinv = (double)rif;
             if(!(r > 0.0)) continue;  // r^2 below FP32's range: coincident for the force
             ++n_pairs;
-            const double4 tj = ldg4(&S.thermo[j]);
+            double4 sj = make_double4(0, 0, 0, 0);
+            if(TYPE != SPHGPU_GSPH) sj = ldg4(&S.visc[j]);
             const T rT = (T)r;
             const T rinvT = (T)rinv;
             const V3<T> rv{(T)d.x, (T)d.y, (T)d.z};
-            const KernH<T> khj(P.kernel, (T)hj);
+            const KernH<T> khj(KER == ANY_KERNEL ? P.kernel : KER, (T)hj);
             const T ci_ = khi.dwc(rT, rinvT);
             const T cj_ = khj.dwc(rT, rinvT);
             const V3<T> dwi{rv.x * ci_, rv.y * ci_, rv.z * ci_};
@@ -449,7 +473,6 @@ __global__ void __launch_bounds__(FBLK, (TYPE == SPHGPU_DISPH ? 3 : 4)) k_force_
                     continue;
                 }
             }
-            const double4 sj = ldg4(&S.visc[j]);
             const V3<T> dwij{(dwi.x + dwj.x) * T(0.5), (dwi.y + dwj.y) * T(0.5), (dwi.z + dwj.z) * T(0.5)};
             const V3<T> vij{(T)(vi.x - vj.x), (T)(vi.y - vj.y), (T)(vi.z - vj.z)};
             // artificial viscosity (src/fluid_force.cpp:88-106)
@@ -939,16 +962,17 @@ unsigned force_grid(int n, int threads = FBLK)
     return (unsigned)std::max<long long>(1, std::min<long long>(blocks, 148LL * 8 * 4 * (FBLK / threads)));
 }
 
-template <int TYPE, int MODE>
-void launch_force_mixed(sphgpu_ctx* c, MlpPairs mp, Harvest hv, Subset sub)
-{
-    k_force_mixed<GROUP, TYPE, MODE><<<force_grid(c->n), FBLK, 0, c->stream>>>(
-        c->dp, c->s, c->n, c->d_plist, c->d_pcount, (int)c->pcap, c->d_dt, c->d_status, mp, hv, c->d_accabs, sub);
-}
-
 template <int TYPE, int MODE, int KER>
-void launch_force_form(sphgpu_ctx* c, MlpPairs mp, Harvest hv, Subset sub)
+void launch_force_form(sphgpu_ctx* c, bool mixed, MlpPairs mp, Harvest hv, Subset sub)
 {
+    if(mixed) {
+        constexpr int ker = TYPE == SPHGPU_DISPH ? KER : ANY_KERNEL;
+        auto* k = c->prm.periodic ? k_force_mixed<GROUP, TYPE, ker, true, MODE>
+                                  : k_force_mixed<GROUP, TYPE, ker, false, MODE>;
+        k<<<force_grid(c->n), FBLK, 0, c->stream>>>(c->dp, c->s, c->n, c->d_plist, c->d_pcount, (int)c->pcap, c->d_dt,
+                                                    c->d_status, mp, hv, c->d_accabs, sub);
+        return;
+    }
     auto* k = c->prm.periodic ? k_force64<GROUP, TYPE, KER, true, MODE> : k_force64<GROUP, TYPE, KER, false, MODE>;
     constexpr int threads = force64_threads(TYPE);
     k<<<force_grid(sub.idx ? sub.n : c->n, threads), threads, 0, c->stream>>>(
@@ -958,10 +982,9 @@ void launch_force_form(sphgpu_ctx* c, MlpPairs mp, Harvest hv, Subset sub)
 template <int TYPE, int MODE>
 void launch_force_type(sphgpu_ctx* c, bool mixed, MlpPairs mp, Harvest hv, Subset sub)
 {
-    if(mixed) launch_force_mixed<TYPE, MODE>(c, mp, hv, sub);
-    else if(c->prm.kernel == SPHGPU_WENDLAND) launch_force_form<TYPE, MODE, SPHGPU_WENDLAND>(c, mp, hv, sub);
-    else if(c->prm.kernel == SPHGPU_GAUSSIAN) launch_force_form<TYPE, MODE, SPHGPU_GAUSSIAN>(c, mp, hv, sub);
-    else launch_force_form<TYPE, MODE, SPHGPU_CUBIC_SPLINE>(c, mp, hv, sub);
+    if(c->prm.kernel == SPHGPU_WENDLAND) launch_force_form<TYPE, MODE, SPHGPU_WENDLAND>(c, mixed, mp, hv, sub);
+    else if(c->prm.kernel == SPHGPU_GAUSSIAN) launch_force_form<TYPE, MODE, SPHGPU_GAUSSIAN>(c, mixed, mp, hv, sub);
+    else launch_force_form<TYPE, MODE, SPHGPU_CUBIC_SPLINE>(c, mixed, mp, hv, sub);
 }
 
 template <int MODE>

@@ -477,24 +477,17 @@ __global__ void __launch_bounds__(PBLK, PRE_BLOCKS) k_pre(DevParams P, DevState 
     block_count(&st->pre_list, n_list);
 }
 
-// The sweep's pair test and FP32 distance: true when r < h exactly as the
-// reference decides it (root_lt on the unfused FP64 r^2).
-__device__ __forceinline__ bool sweep_r(double r2, double h, float& r)
-{
-    if(!root_lt(r2, h)) return false;
-    const float r2f = (float)r2;
-    r = r2f > 0.f ? r2f * rsqrtf(r2f) : 0.f;
-    return true;
-}
-
 // The mixed form: pair arithmetic and sums in FP32.  A kernel of its own: the
 // smoothing length follows the rounding of the FP32 sums, and with it which
-// pairs lie inside, so its operations stay as they are (the FP64 kernel's
-// masked evaluation gained 10 % here and moved h by 1e-7, a handful of pairs
-// across the kernel's edge in a million particles).  Resident blocks measured:
-// disph 3 (2: 27.3 -> 34.5 ms on the 8.8 M sphere), ssph 4.
-template <int G, int TYPE>
-__global__ void __launch_bounds__(PBLK, (TYPE == SPHGPU_SSPH ? 4 : 3)) k_pre_mixed(DevParams P, DevState S, int n, const int* __restrict__ list,
+// pairs lie inside (a move of h by 1e-7 takes a handful of pairs in a million
+// particles across the kernel's edge), so its operations and their fusing are
+// spelt out and stay as they are.  What changed around them: two candidates are
+// evaluated and masked per iteration, the box and the kernel function are
+// compile-time, and two resident blocks leave registers for both candidates
+// (1.1 M disph sphere 3.00 -> 2.75 ms, 131 K shear layer 0.477 -> 0.398, 493 K
+// ssph sphere 0.69 -> 0.59, 1 M gsph tube 1.54 -> 1.30, gdisph 1.92 -> 1.47).
+template <int G, int TYPE, int KER, bool PER>
+__global__ void __launch_bounds__(PBLK, PRE_BLOCKS) k_pre_mixed(DevParams P, DevState S, int n, const int* __restrict__ list,
                                               const int* __restrict__ count, int cap, const double* __restrict__ dtp,
                                               double* __restrict__ hvs, DevStatus* __restrict__ st, DevTree Tr,
                                               double skin_delta, int* __restrict__ scratch, int scap)
@@ -544,33 +537,13 @@ __global__ void __launch_bounds__(PBLK, (TYPE == SPHGPU_SSPH ? 4 : 3)) k_pre_mix
             for(int it = 0; it < 10; ++it) {
                 const double hb = h;
                 T d = 0, dd = 0;
-                const KernH<T> kh(P.kernel, (T)h);
+                const KernF<KER> kh((T)h);
+                const Within in(h);
                 const bool exact = skin_delta > 0.0 && !(h < sml0 - skin_delta);
                 const double hk = h * (1.0 + 4e-4), keep2 = hk * hk;
                 nk = 0;
-                auto visit = [&](const double4& pj, int jc) {
-                    const double r2 = abs2x(rij(P, pi.x, pi.y, pi.z, pj.x, pj.y, pj.z));
-                    if constexpr(keep) {
-                        if(r2 < keep2) srow[lane + G * nk++] = jc;
-                    }
-                    T rT;
-                    if(sweep_r(r2, h, rT) && (!exact || gather_member(P, Tr, pi.x, pi.y, pi.z, sml0, skin_delta, jc, r2))) {
-                        ++n_newton;
-                        const T w = kh.w(rT);
-                        const T dh = kh.dhw(rT);
-                        if(disph) {
-                            d += w;
-                            dd += dh;
-                        } else {
-                            d += (T)pj.w * w;
-                            dd += (T)pj.w * dh;
-                        }
-                    }
-                };
-                // two candidates per iteration (the same per-lane order), their
-                // indices fetched an iteration ahead: two position loads in
-                // flight, neither waiting on the list load (8.78 M sphere:
-                // 34.9 -> 32.5 ms FP64)
+                // two candidates per iteration (the same per-lane order), both
+                // evaluated; a sum keeps its value where the mask is off
                 int ja = lane < cnt ? __ldg(&li[lane]) : 0;
                 int jb = lane + G < cnt ? __ldg(&li[lane + G]) : 0;
                 n_cand += lane < cnt ? (unsigned)((cnt - lane + G - 1) / G) : 0u;
@@ -581,8 +554,32 @@ __global__ void __launch_bounds__(PBLK, (TYPE == SPHGPU_SSPH ? 4 : 3)) k_pre_mix
                     if(k + 3 * G < cnt) jb = __ldg(&li[k + 3 * G]);
                     const double4 pa = ldg4(&S.pos[ca]);
                     const double4 pb = ldg4(&S.pos[cb]);
-                    visit(pa, ca);
-                    if(two) visit(pb, cb);
+                    const double r2a = abs2x(offset_of<PER>(P, pi, pa)), r2b = abs2x(offset_of<PER>(P, pi, pb));
+                    if constexpr(keep) {
+                        if(r2a < keep2) srow[lane + G * nk++] = ca;
+                        if(two && r2b < keep2) srow[lane + G * nk++] = cb;
+                    }
+                    bool ia = in.sure(r2a), ib = two && in.sure(r2b);
+                    const bool ua = in.unsure(r2a), ub = two && in.unsure(r2b);
+                    if(ua || ub || (exact && (ia || ib))) {  // rare
+                        if(ua) ia = sqrt(r2a) < h;
+                        if(ub) ib = sqrt(r2b) < h;
+                        if(exact && ia) ia = gather_member(P, Tr, pi.x, pi.y, pi.z, sml0, skin_delta, ca, r2a);
+                        if(exact && ib) ib = gather_member(P, Tr, pi.x, pi.y, pi.z, sml0, skin_delta, cb, r2b);
+                    }
+                    n_newton += (ia ? 1u : 0u) + (ib ? 1u : 0u);
+                    auto add = [&](double r2, bool inside, T mj) {
+                        const float r2f = (float)r2;
+                        const T rT = r2f > 0.f ? r2f * rsqrtf(r2f) : 0.f;
+                        const T w = kh.w(rT);
+                        const T dh = kh.dhw(rT);
+                        const T dn = disph ? __fadd_rn(d, w) : fmaf(mj, w, d);
+                        const T ddn = disph ? __fadd_rn(dd, dh) : fmaf(mj, dh, dd);
+                        d = inside ? dn : d;
+                        dd = inside ? ddn : dd;
+                    };
+                    add(r2a, ia, (T)pa.w);
+                    add(r2b, ib, (T)pb.w);
                 }
                 const double ds = (double)group_sum<G>(d), dds = (double)group_sum<G>(dd);
                 const double h3 = h * h * h;
@@ -601,7 +598,8 @@ __global__ void __launch_bounds__(PBLK, (TYPE == SPHGPU_SSPH ? 4 : 3)) k_pre_mix
         }
 
         // ---- 2. fused pass over {r < h}
-        const KernH<T> kh(P.kernel, (T)h);
+        const KernF<KER> kh((T)h);
+        const Within in(h);
         T dens = 0, dhd = 0, ni = 0, pres = 0, dhp = 0, dhn = 0;
         T divv = 0, rx = 0, ry = 0, rz = 0;
         T gd[3] = {0, 0, 0}, gu[3] = {0, 0, 0}, gv[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
@@ -613,98 +611,122 @@ __global__ void __launch_bounds__(PBLK, (TYPE == SPHGPU_SSPH ? 4 : 3)) k_pre_mix
         n_list += lane < cnt ? (unsigned)((cnt - lane + G - 1) / G) : 0u;
         const bool kept = keep && conv;
         n_cand += kept ? (unsigned)nk : (lane < cnt ? (unsigned)((cnt - lane + G - 1) / G) : 0u);
-        auto visit = [&](const double4& pj, int j) {
-            const Vec3d dv = rij(P, pi.x, pi.y, pi.z, pj.x, pj.y, pj.z);
-            const double r2 = abs2x(dv);
+        // one candidate, evaluated and masked (`use`: it is in the list): a sum
+        // keeps its value where the mask is off
+        struct Pair {
+            Vec3d dv;
+            double r2;
+            bool in;
+            double4 v, t;
+        };
+        auto load = [&](const double4& pj, int j, bool use) {
+            Pair q;
+            q.dv = offset_of<PER>(P, pi, pj);
+            q.r2 = abs2x(q.dv);
             // the set predicate in FP64, the distance in FP32
-            if(!root_lt(r2, h)) return;
-            const float r2f = (float)r2;
-            const float rif = r2f > 0.f ? rsqrtf(r2f) : 0.f;
-            const double r = (double)(r2f * rif), rinv = (double)rif;
-            if(exact && !gather_member(P, Tr, pi.x, pi.y, pi.z, sml0, skin_delta, j, r2)) return;
-            ++nn;
+            q.in = use && in.sure(q.r2);
+            const bool unsure = use && in.unsure(q.r2);
+            if(unsure || (exact && q.in)) {  // rare
+                if(unsure) q.in = sqrt(q.r2) < h;
+                if(exact && q.in) q.in = gather_member(P, Tr, pi.x, pi.y, pi.z, sml0, skin_delta, j, q.r2);
+            }
             // coherent loads: this kernel writes vel.w and thermo.x, .y of every
             // particle (the components read here, velocity, u and c_s, it
             // does not change)
-            const double4 vj = S.vel[j];
-            const double4 tj = S.thermo[j];
+            q.v = q.t = make_double4(0, 0, 0, 0);
+            if(q.in) {
+                q.v = S.vel[j];
+                q.t = S.thermo[j];
+            }
+            return q;
+        };
+        auto add = [&](const double4& pj, int j, const Pair& q) {
+            const float r2f = (float)q.r2;
+            const float rif = r2f > 0.f ? rsqrtf(r2f) : 0.f;
+            const double r = (double)(r2f * rif), rinv = (double)rif;
+            auto put = [&](T& sum, T with) { sum = q.in ? with : sum; };
+            nn += q.in ? 1 : 0;
             const T rT = (T)r;
             const T w = kh.w(rT);
             const T mj = (T)pj.w;
             if(disph) {
                 const T dh = kh.dhw(rT);
-                const T uj = (T)tj.z;
-                dens += mj * w;
-                ni += w;
-                pres += mj * uj * w;
-                dhp += mj * uj * dh;
-                dhn += dh;
+                const T uj = (T)q.t.z;
+                put(dens, fmaf(mj, w, dens));
+                put(ni, ni + w);
+                put(pres, fmaf(mj * uj, w, pres));
+                put(dhp, fmaf(mj * uj, dh, dhp));
+                put(dhn, dhn + dh);
             } else {
-                dens += mj * w;
-                if(!gsph) dhd += mj * kh.dhw(rT);
+                put(dens, TYPE == SPHGPU_SSPH ? __fadd_rn(dens, __fmul_rn(mj, w)) : fmaf(mj, w, dens));
+                if(!gsph) put(dhd, fmaf(mj, kh.dhw(rT), dhd));
             }
-            if(i != j) {
-                const double vr = dv.x * (vi.x - vj.x) + dv.y * (vi.y - vj.y) + dv.z * (vi.z - vj.z);
+            {
+                const double vr = q.dv.x * (vi.x - q.v.x) + q.dv.y * (vi.y - q.v.y) + q.dv.z * (vi.z - q.v.z);
                 // coincident particles (r = 0): the reference's vr / r is
                 // 0 / 0, a NaN that never raises v_sig (+-inf if r underflowed)
-                const double v = r > 0.0 ? ti.w + tj.w - 3.0 * vr * rinv
+                const double v = r > 0.0 ? ti.w + q.t.w - 3.0 * vr * rinv
                                          : (vr < 0.0 ? (double)INFINITY : -(double)INFINITY);
-                if(v > vsig) vsig = v;
+                if(q.in && i != j && v > vsig) vsig = v;
             }
             if(need_av || need_grad) {
-                const T c = kh.dwc(rT, (T)rinv);
-                const T dwx = (T)dv.x * c, dwy = (T)dv.y * c, dwz = (T)dv.z * c;
-                const T vx = (T)(vi.x - vj.x), vy = (T)(vi.y - vj.y), vz = (T)(vi.z - vj.z);
+                const T c = TYPE == SPHGPU_DISPH ? kh.k.dwc(rT, (T)rinv) : kh.dwc(rT, (T)rinv);
+                const T dwx = (T)q.dv.x * c, dwy = (T)q.dv.y * c, dwz = (T)q.dv.z * c;
+                const T vx = (T)(vi.x - q.v.x), vy = (T)(vi.y - q.v.y), vz = (T)(vi.z - q.v.z);
                 if(need_av) {
-                    const T wgt = av_energy ? mj * (T)tj.z : mj;
-                    divv -= wgt * (vx * dwx + vy * dwy + vz * dwz);
-                    rx += (vy * dwz - vz * dwy) * wgt;
-                    ry += (vz * dwx - vx * dwz) * wgt;
-                    rz += (vx * dwy - vy * dwx) * wgt;
+                    const T wgt = av_energy ? mj * (T)q.t.z : mj;
+                    put(divv, fmaf(-wgt, vx * dwx + vy * dwy + vz * dwz, divv));
+                    put(rx, fmaf(vy * dwz - vz * dwy, wgt, rx));
+                    put(ry, fmaf(vz * dwx - vx * dwz, wgt, ry));
+                    put(rz, fmaf(vx * dwy - vy * dwx, wgt, rz));
                 }
                 if(need_grad) {
-                    const T du = mj * (T)(tj.z - ti.z);
-                    gd[0] += dwx * mj;
-                    gd[1] += dwy * mj;
-                    gd[2] += dwz * mj;
-                    gu[0] += dwx * du;
-                    gu[1] += dwy * du;
-                    gu[2] += dwz * du;
+                    const T du = mj * (T)(q.t.z - ti.z);
+                    put(gd[0], fmaf(dwx, mj, gd[0]));
+                    put(gd[1], fmaf(dwy, mj, gd[1]));
+                    put(gd[2], fmaf(dwz, mj, gd[2]));
+                    put(gu[0], fmaf(dwx, du, gu[0]));
+                    put(gu[1], fmaf(dwy, du, gu[1]));
+                    put(gu[2], fmaf(dwz, du, gu[2]));
                     // dv[k] += dw * (m_j (v_j[k] - v_i[k]))
                     const T m0 = -mj * vx, m1 = -mj * vy, m2 = -mj * vz;
-                    gv[0] += dwx * m0;
-                    gv[1] += dwy * m0;
-                    gv[2] += dwz * m0;
-                    gv[3] += dwx * m1;
-                    gv[4] += dwy * m1;
-                    gv[5] += dwz * m1;
-                    gv[6] += dwx * m2;
-                    gv[7] += dwy * m2;
-                    gv[8] += dwz * m2;
+                    put(gv[0], fmaf(dwx, m0, gv[0]));
+                    put(gv[1], fmaf(dwy, m0, gv[1]));
+                    put(gv[2], fmaf(dwz, m0, gv[2]));
+                    put(gv[3], fmaf(dwx, m1, gv[3]));
+                    put(gv[4], fmaf(dwy, m1, gv[4]));
+                    put(gv[5], fmaf(dwz, m1, gv[5]));
+                    put(gv[6], fmaf(dwx, m2, gv[6]));
+                    put(gv[7], fmaf(dwy, m2, gv[7]));
+                    put(gv[8], fmaf(dwz, m2, gv[8]));
                 }
             }
         };
         if(kept) {
             // the lane's kept candidates, in its own order (the same sums)
-            int m = 0;
-            for(; m + 1 < nk; m += 2) {
-                const int ca = srow[lane + G * m], cb = srow[lane + G * (m + 1)];
+            for(int m = 0; m < nk; m += 2) {
+                const bool two = m + 1 < nk;
+                const int ca = srow[lane + G * m], cb = two ? srow[lane + G * (m + 1)] : ca;
                 const double4 pa = ldg4(&S.pos[ca]);
                 const double4 pb = ldg4(&S.pos[cb]);
-                visit(pa, ca);
-                visit(pb, cb);
-            }
-            if(m < nk) {
-                const int ca = srow[lane + G * m];
-                visit(ldg4(&S.pos[ca]), ca);
+                const Pair qa = load(pa, ca, true), qb = load(pb, cb, two);
+                add(pa, ca, qa);
+                add(pb, cb, qb);
             }
         } else {
-            // the next candidate's index is fetched one iteration ahead
-            int jn = lane < cnt ? __ldg(&li[lane]) : 0;
-            for(int k = lane; k < cnt; k += G) {
-                const int j = jn;
-                if(k + G < cnt) jn = __ldg(&li[k + G]);
-                visit(ldg4(&S.pos[j]), j);
+            // the next candidates' indices are fetched one iteration ahead
+            int ja = lane < cnt ? __ldg(&li[lane]) : 0;
+            int jb = lane + G < cnt ? __ldg(&li[lane + G]) : 0;
+            for(int k = lane; k < cnt; k += 2 * G) {
+                const int ca = ja, cb = jb;
+                const bool two = k + G < cnt;
+                if(k + 2 * G < cnt) ja = __ldg(&li[k + 2 * G]);
+                if(k + 3 * G < cnt) jb = __ldg(&li[k + 3 * G]);
+                const double4 pa = ldg4(&S.pos[ca]);
+                const double4 pb = ldg4(&S.pos[cb]);
+                const Pair qa = load(pa, ca, true), qb = load(pb, cb, two);
+                add(pa, ca, qa);
+                add(pb, cb, qb);
             }
         }
         n_pairs += (unsigned)nn;
@@ -889,14 +911,17 @@ void launch_pre_kernel(sphgpu_ctx* c, K* k)
 template <int TYPE, int KER>
 void launch_pre_form(sphgpu_ctx* c)
 {
-    launch_pre_kernel(c, c->prm.periodic ? k_pre<GROUP, TYPE, KER, true> : k_pre<GROUP, TYPE, KER, false>);
+    if(c->prm.precision == SPHGPU_MIXED) {
+        launch_pre_kernel(c, c->prm.periodic ? k_pre_mixed<GROUP, TYPE, KER, true> : k_pre_mixed<GROUP, TYPE, KER, false>);
+    } else {
+        launch_pre_kernel(c, c->prm.periodic ? k_pre<GROUP, TYPE, KER, true> : k_pre<GROUP, TYPE, KER, false>);
+    }
 }
 
 template <int TYPE>
 void launch_pre(sphgpu_ctx* c)
 {
-    if(c->prm.precision == SPHGPU_MIXED) launch_pre_kernel(c, k_pre_mixed<GROUP, TYPE>);
-    else if(c->prm.kernel == SPHGPU_WENDLAND) launch_pre_form<TYPE, SPHGPU_WENDLAND>(c);
+    if(c->prm.kernel == SPHGPU_WENDLAND) launch_pre_form<TYPE, SPHGPU_WENDLAND>(c);
     else if(c->prm.kernel == SPHGPU_GAUSSIAN) launch_pre_form<TYPE, SPHGPU_GAUSSIAN>(c);
     else launch_pre_form<TYPE, SPHGPU_CUBIC_SPLINE>(c);
 }
