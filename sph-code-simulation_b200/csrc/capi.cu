@@ -574,6 +574,7 @@ int sphgpu_destroy(sphgpu_ctx* c)
     free_all(c);
     if(c->d_mlp) cudaFree(c->d_mlp);
     if(c->d_mlp_master) cudaFree(c->d_mlp_master);
+    if(c->d_mlp_work) cudaFree(c->d_mlp_work);
     if(c->d_relax) cudaFree(c->d_relax);
     if(c->d_tcount) cudaFree(c->d_tcount);
     if(c->d_flist_flags) cudaFree(c->d_flist_flags);

@@ -110,6 +110,9 @@ struct sphgpu_ctx {
     // learned Riemann guess (BF16 weights + FP32 biases on device)
     void* d_mlp = nullptr;            // BF16 / FP32 image read by the kernels
     float* d_mlp_master = nullptr;    // FP32 master parameters + Adam moments
+    // workspace of the calls on host states (mlp.cu), kept up to a bound
+    void* d_mlp_work = nullptr;
+    size_t mlp_work_bytes = 0;
     // deferred pairs of the learned path: rows (features, pair keys, network
     // output, sort buffers) and per-particle row ranges, in one allocation
     void* d_mlp_defer = nullptr;

@@ -60,3 +60,21 @@ def test_adam_steps_from_the_gradient(gpu, M):
     np.testing.assert_allclose(step, -lr * np.sign(grad[big]), atol=2e-4 * lr + 2.0 ** -24)
     y_ref, _ = M.forward(after, M.features(states), emulate_bf16=True)
     assert np.max(np.abs(y - y_ref)) < 2e-2
+
+
+def test_workspace_kept_between_calls(gpu, M):
+    """Calls of rising and falling size on one context, past the size whose
+    workspace is kept (64 MB, 84 bytes a row): the outputs of a fresh context."""
+    with gpu.Simulation(gpu.config_params("tube_gsph")) as sim:
+        sim.mlp_init(3)
+        for n in (100, 900_000, 40_000, 7):
+            states = M.random_states(n, seed=n)
+            y = sim.mlp_predict(states)
+            loss, grad = sim.mlp_train(states, states[:, 2], epochs=0)
+            with gpu.Simulation(gpu.config_params("tube_gsph")) as fresh:
+                fresh.mlp_init(3)
+                np.testing.assert_array_equal(y, fresh.mlp_predict(states))
+                loss_f, grad_f = fresh.mlp_train(states, states[:, 2], epochs=0)
+            # sums over blocks in any order: 148 FP32 additions
+            assert loss == pytest.approx(loss_f, rel=148 * 2.0 ** -24)
+            assert np.max(np.abs(grad - grad_f)) <= 148 * 2.0 ** -24 * np.max(np.abs(grad_f))
