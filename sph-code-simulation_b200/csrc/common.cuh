@@ -508,7 +508,7 @@ __device__ __forceinline__ unsigned group_mask()
 {
     if(G == 32) return FULL_MASK;
     const unsigned lane = threadIdx.x & 31u;
-    return ((1u << G) - 1u) << (lane & ~(unsigned)(G - 1));
+    return (0xffffffffu >> (32 - G)) << (lane & ~(unsigned)(G - 1));
 }
 template <int G, typename T>
 __device__ __forceinline__ T group_sum(T v)

@@ -39,7 +39,11 @@ namespace sphgpu {
 namespace {
 
 constexpr int LBLK = 256;
-constexpr int LG = 8;  // lanes per particle (8: 1.57 ms vs 1.71 ms with 4, shear 1 M)
+// Lanes per particle.  A warp to one particle reads its list in coalesced rows
+// and appends to fewer rows at once than 8 lanes did (which in turn beat 4): 4 K
+// sphere 41 -> 20 us, 493 K 863 -> 821, 298 K shear layer 527 -> 508, 57 K gdisph
+// tube 69 -> 66 (each with the finalise pass).
+constexpr int LG = 32;
 
 __global__ void k_save_radius(const DevState S, int n, double* __restrict__ rs)
 {
@@ -91,7 +95,7 @@ __global__ void __launch_bounds__(LBLK, 5) k_flist(DevParams P, DevState S, int 
             return true;
         };
         auto compact = [&](bool own, int j) {
-            const unsigned m = (__ballot_sync(gmask, own) >> gbase) & ((1u << G) - 1u);
+            const unsigned m = (__ballot_sync(gmask, own) >> gbase) & (0xffffffffu >> (32 - G));
             if(own) {
                 const int pos = oc + __popc(m & ((1u << lane) - 1u));
                 if(pos < pcap) row[pos] = j;
@@ -118,23 +122,28 @@ __global__ void __launch_bounds__(LBLK, 5) k_flist(DevParams P, DevState S, int 
 }
 
 // Appended entries: sorted by index and moved behind the own entries.  A warp
-// takes 32 rows: a few entries are sorted by the row's own lane, longer tails
+// takes up to 32 rows: a few entries are sorted by the row's own lane, longer tails
 // by the whole warp, every entry to its rank (indices are unique).  In a
 // graded sphere the centre's rows are appended to by a hundred neighbours and
 // more; one lane's insertion sort over global memory was then the pass.
 constexpr int FSHORT = 4;      // entries a lane sorts by itself, in registers
 constexpr int FBUF = 512;      // entries a warp ranks from shared memory
 constexpr int FWARPS = 4;
+// Rows of one warp: 32 in large sets, where the short tails' lanes are the work;
+// fewer while that leaves under 32 warps per SM, as a warp ranks its long tails
+// one after the other (4 K sphere: 64 -> 10 us; 28 K with 64 warps per SM wanted
+// 102 -> 97 but 17 K 37 -> 42).
+constexpr int FFILL = 148 * 32;
 __global__ void __launch_bounds__(FWARPS * 32) k_flist_finalize(int n, int* __restrict__ plist,
                                                                int* __restrict__ pcount,
-                                                               const int* __restrict__ tcount, int pcap,
+                                                               const int* __restrict__ tcount, int pcap, int per,
                                                                int fatal_limit, int* __restrict__ flags)
 {
     __shared__ int s_buf[FWARPS][FBUF];
     const int lane = threadIdx.x & 31;
     int* buf = s_buf[threadIdx.x >> 5];
-    const int i = blockIdx.x * FWARPS * 32 + threadIdx.x;
-    const bool valid = i < n;
+    const int i = (blockIdx.x * FWARPS + (threadIdx.x >> 5)) * per + lane;
+    const bool valid = lane < per && i < n;
     const int oc = valid ? pcount[i] : 0, tc = valid ? tcount[i] : 0;
     const long long tot = (long long)oc + tc;
     const bool fits = tot <= pcap;
@@ -214,7 +223,9 @@ int build_force_lists(sphgpu_ctx* c)
     k_flist<LG><<<grid, LBLK, 0, st>>>(c->dp, c->s, n, c->d_glist, c->d_gcount, (int)c->gcap, c->d_rsearch,
                                        c->d_plist, c->d_pcount, c->d_tcount, (int)c->pcap, c->d_flist_flags,
                                        c->t, c->skin_valid ? c->skin_delta_now : 0.0);
-    k_flist_finalize<<<grid_for(n, FWARPS * 32), FWARPS * 32, 0, st>>>(n, c->d_plist, c->d_pcount, c->d_tcount, (int)c->pcap,
+    int per = 32;
+    while(per > 1 && n / per < FFILL) per /= 2;
+    k_flist_finalize<<<grid_for(n, FWARPS * per), FWARPS * 32, 0, st>>>(n, c->d_plist, c->d_pcount, c->d_tcount, (int)c->pcap, per,
                                                         c->prm.neighbor_number * 1000, c->d_flist_flags);
     SPHGPU_LAUNCH_CHECK(c, "force lists");
     stage_end(c, SPHGPU_T_PAIR_WALK, 2);
