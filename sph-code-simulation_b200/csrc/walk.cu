@@ -16,8 +16,8 @@
 // own particle in FP32 with rigorously rounded thresholds (certainly inside /
 // certainly outside / a thin band at the radius), and only band pairs run the
 // reference's FP64 test, with the box tests replayed up the parent chain for
-// pairs on the radius.  Warps whose particles straddle a large octant
-// boundary are split into compact sub-groups walked one after another.
+// pairs on the radius.  Windows whose particles straddle a large octant
+// boundary are split into compact sub-groups, each walked by a warp of its own.
 //
 // Per-lane walk (k_walk, the fallback and cross-check): each lane keeps one
 // bit per tree level: bit L says "my box test passed at the current level-L
