@@ -39,11 +39,17 @@ namespace sphgpu {
 namespace {
 
 constexpr int LBLK = 256;
-// Lanes per particle.  A warp to one particle reads its list in coalesced rows
-// and appends to fewer rows at once than 8 lanes did (which in turn beat 4): 4 K
-// sphere 41 -> 20 us, 493 K 863 -> 821, 298 K shear layer 527 -> 508, 57 K gdisph
-// tube 69 -> 66 (each with the finalise pass).
-constexpr int LG = 32;
+// Lanes per particle: 8, and a whole warp from neighbor_number LG_WIDE_K on.  A
+// list holds about twice neighbor_number entries and an iteration takes two of
+// them per lane, so short lists leave a warp's lanes idle: even at K = 64 and 80
+// (300 K sphere 314 -> 302 us, shear layer 334 -> 344), 5 % faster at 96 (449 ->
+// 423, 401 -> 384).  Both passes, 8 -> 32 lanes: K = 128 1.1 M
+// sphere 1.81 -> 1.65 ms, 1 M shear layer 1.67 -> 1.55, 4.2 M sphere 6.76 -> 6.04,
+// 4 K sphere 38 -> 30 us; K = 50 1 M gsph tube 0.695 -> 0.797, 1 M ssph sphere
+// 0.703 -> 0.780 (16 lanes lie between; 4 are slower than 8).
+constexpr int LG = 8;
+constexpr int LG_WIDE = 32;
+constexpr int LG_WIDE_K = 96;
 
 __global__ void k_save_radius(const DevState S, int n, double* __restrict__ rs)
 {
@@ -218,11 +224,13 @@ int build_force_lists(sphgpu_ctx* c)
     stage_begin(c, SPHGPU_T_PAIR_WALK);
     SPHGPU_CUDA(c, cudaMemsetAsync(c->d_tcount, 0, sizeof(int) * (size_t)n, st));
     SPHGPU_CUDA(c, cudaMemsetAsync(c->d_flist_flags, 0, 3 * sizeof(int), st));
-    const long long gpb = LBLK / LG;
+    const bool wide = c->prm.neighbor_number >= LG_WIDE_K;
+    const long long gpb = LBLK / (wide ? LG_WIDE : LG);
     const unsigned grid = (unsigned)std::max<long long>(1, std::min<long long>((n + gpb - 1) / gpb, 148LL * 8 * 4));
-    k_flist<LG><<<grid, LBLK, 0, st>>>(c->dp, c->s, n, c->d_glist, c->d_gcount, (int)c->gcap, c->d_rsearch,
-                                       c->d_plist, c->d_pcount, c->d_tcount, (int)c->pcap, c->d_flist_flags,
-                                       c->t, c->skin_valid ? c->skin_delta_now : 0.0);
+    auto* k = wide ? k_flist<LG_WIDE> : k_flist<LG>;
+    k<<<grid, LBLK, 0, st>>>(c->dp, c->s, n, c->d_glist, c->d_gcount, (int)c->gcap, c->d_rsearch, c->d_plist,
+                             c->d_pcount, c->d_tcount, (int)c->pcap, c->d_flist_flags, c->t,
+                             c->skin_valid ? c->skin_delta_now : 0.0);
     int per = 32;
     while(per > 1 && n / per < FFILL) per /= 2;
     k_flist_finalize<<<grid_for(n, FWARPS * per), FWARPS * 32, 0, st>>>(n, c->d_plist, c->d_pcount, c->d_tcount, (int)c->pcap, per,
