@@ -91,17 +91,70 @@ __device__ __forceinline__ T vl_newton_step(T p, T ul, T pl, T vl, T cl, T ur, T
     return fmax(T(1e-25), p);
 }
 
+// The same update and the final u* in FP64 with an operation policy
+// (rounded.cuh); every quotient and root is rounded as the general operations'.
+template <typename Op>
+__device__ __forceinline__ double vl_step(Op& op, double p, double ul, double pl, double vl, double cl, double ur,
+                                          double pr, double vr, double cr, double g1, double g2)
+{
+    const double wl = cl * op.root(1.0 + op.div0(g1 * (p - pl), pl));
+    const double wr = cr * op.root(1.0 + op.div0(g1 * (p - pr), pr));
+    double zl = 4.0 * vl * wl * wl;
+    zl = op.div(-zl * wl, zl - g2 * (p - pl));
+    double zr = 4.0 * vr * wr * wr;
+    zr = op.div(zr * wr, zr - g2 * (p - pr));
+    const double usl = ul - op.div0(p - pl, wl);
+    const double usr = ur + op.div0(p - pr, wr);
+    p = p + op.div0((usr - usl) * (zl * zr), zr - zl);
+    return fmax(1e-25, p);
+}
+template <typename Op>
+__device__ __forceinline__ double vl_ustar_of(Op& op, double p, double ul, double pl, double cl, double ur, double pr,
+                                              double cr, double g1)
+{
+    const double wl = cl * op.root(1.0 + op.div0(g1 * (p - pl), pl));
+    const double wr = cr * op.root(1.0 + op.div0(g1 * (p - pr), pr));
+    const double usl = ul - op.div0(p - pl, wl);
+    const double usr = ur + op.div0(p - pr, wr);
+    return 0.5 * (usl + usr);
+}
+
+// The learned start's steps: branch-free operations first, the general ones (out
+// of line) where an intermediate leaves their range.  125 K blast, both passes:
+// 2.17 -> 2.05 ms.  The mixed form's plain solver keeps the general ones for its
+// one FP64 step, where both take the same time (1 M tube 3.84 ms).
+__device__ __noinline__ double vl_step_ieee(double p, double ul, double pl, double vl, double cl, double ur, double pr,
+                                            double vr, double cr, double g1, double g2)
+{
+    Ieee op;
+    return vl_step(op, p, ul, pl, vl, cl, ur, pr, vr, cr, g1, g2);
+}
+__device__ __forceinline__ double vl_step_quick(double p, double ul, double pl, double vl, double cl, double ur,
+                                                double pr, double vr, double cr, double g1, double g2)
+{
+    Quick op;
+    const double q = vl_step(op, p, ul, pl, vl, cl, ur, pr, vr, cr, g1, g2);
+    return op.bad ? vl_step_ieee(p, ul, pl, vl, cl, ur, pr, vr, cr, g1, g2) : q;
+}
 // Final wave speeds and u* at p (src/gsph/g_fluid_force.cpp:285-298), FP64.
+__device__ __noinline__ double vl_ustar_ieee(double p, double ul, double pl, double cl, double ur, double pr,
+                                             double cr, double g1)
+{
+    Ieee op;
+    return vl_ustar_of(op, p, ul, pl, cl, ur, pr, cr, g1);
+}
+__device__ __forceinline__ double vl_ustar_quick(double p, double ul, double pl, double cl, double ur, double pr,
+                                                 double cr, double g1)
+{
+    Quick op;
+    const double u = vl_ustar_of(op, p, ul, pl, cl, ur, pr, cr, g1);
+    return op.bad ? vl_ustar_ieee(p, ul, pl, cl, ur, pr, cr, g1) : u;
+}
 __device__ __forceinline__ double vl_ustar(double p, double ul, double pl, double cl, double ur, double pr,
                                            double cr, double g1)
 {
-    double wl = 1.0 + g1 * (p - pl) / pl;
-    wl = cl * sqrt(wl);
-    double wr = 1.0 + g1 * (p - pr) / pr;
-    wr = cr * sqrt(wr);
-    const double usl = ul - (p - pl) / wl;
-    const double usr = ur + (p - pr) / wr;
-    return 0.5 * (usl + usr);
+    Ieee op;
+    return vl_ustar_of(op, p, ul, pl, cl, ur, pr, cr, g1);
 }
 
 // Screen of the learned start: one Newton step from the reference's
@@ -113,7 +166,7 @@ __device__ __noinline__ double learned_screen(double ul, double pl, double vl, d
 {
     double q0 = pr - pl - cr * (ur - ul);
     q0 = fmax(pl + q0 * cl / (cl + cr), 1e-25);
-    q1 = vl_newton_step<double>(q0, ul, pl, vl, cl, ur, pr, vr, cr, g1, g2);
+    q1 = vl_step_quick(q0, ul, pl, vl, cl, ur, pr, vr, cr, g1, g2);
     return fabs(q1 - q0) / q1;
 }
 
@@ -169,13 +222,13 @@ __device__ void riemann_iterative(const double* L, const double* R, double gamma
         bool ok = ch < 1e-10;
         for(int it = 0; !ok && it < budget; ++it) {
             const double pold = p;
-            p = vl_newton_step<double>(p, ul, pl, vl, cl, ur, pr, vr, cr, g1, g2);
+            p = vl_step_quick(p, ul, pl, vl, cl, ur, pr, vr, cr, g1, g2);
             ++iters;
             if(fabs(p - pold) / p < 1e-10) ok = true;
         }
         if(ok) {
             pstar = p;
-            vstar = vl_ustar(p, ul, pl, cl, ur, pr, cr, g1);
+            vstar = vl_ustar_quick(p, ul, pl, cl, ur, pr, cr, g1);
             return;
         }
         fallback = 1;
