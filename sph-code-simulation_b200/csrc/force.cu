@@ -283,12 +283,10 @@ struct Subset {
     int count;
 };
 
-// The mixed form: pair arithmetic in FP32, accumulators in FP64.  Resident
-// blocks per SM measured: disph 3 (17.3 -> 16.0 ms on the 8.8 M sphere), others 4.
 // The mixed form: pair arithmetic in FP32, distances, predicates and sums in
 // FP64.  Bound by the neighbour loads' latency and the conversions between the
-// two precisions (28 % of the pair loop's issue slots lost to loads in flight,
-// the conversions' unit 45 % busy).  The records of the predicate and of the pair
+// two precisions (131 K shear layer, before: 3 of 10 cycles per issue waiting for
+// loads, the conversions' unit 45 % busy).  The records of the predicate and of the pair
 // are loaded together (before, thermo waited for the predicate), the periodic box
 // and, for disph, the kernel function are compile-time, and the resident blocks
 // follow the registers: 1.1 M disph sphere 2.06 -> 1.76 ms, 131 K shear layer
