@@ -614,14 +614,15 @@ __device__ __forceinline__ double dwn_of(double inv)
 template <int KER>
 constexpr double kern_span() { return KER == SPHGPU_CUBIC_SPLINE ? 2.0 : 1.0; }
 
-// van Leer limiter (limiter above) without a branch
+// van Leer limiter (limiter above) without a branch; a product that is not a
+// number (a NaN slope, an infinite one against zero) stays one, as there
 template <typename Op>
 __device__ __forceinline__ double limit(Op& op, double dq1, double dq2)
 {
     const double p = dq1 * dq2;
     const bool some = p > 0.0;
     const double q = op.div(some ? 2.0 * p : 1.0, some ? dq1 + dq2 : 1.0);
-    return p <= 0.0 ? 0.0 : q;
+    return p <= 0.0 ? 0.0 : (some ? q : p);
 }
 
 // riemann_hll with the pair's operations
