@@ -99,7 +99,7 @@ struct Within {
 
 // A pair sum times the factor of h left out of its terms; no pairs, no sum (h of
 // 0 or NaN, from a mass of zero or a bad density guess, has no finite factor).
-__device__ __forceinline__ double scaled(double sum, double factor) { return sum == 0.0 ? 0.0 : sum * factor; }
+__device__ __forceinline__ double scaled(bool some, double sum, double factor) { return some ? sum * factor : 0.0; }
 
 // Two resident blocks per SM (128 registers a thread): with two candidates in
 // flight fewer registers spill (4 blocks of 128 threads: 2.69 -> 2.74 ms on the
@@ -209,7 +209,8 @@ __global__ void __launch_bounds__(PBLK, PRE_BLOCKS) k_pre(DevParams P, DevState 
                         dd += pb.w * sb.dh();
                     }
                 }
-                const double ds = scaled(group_sum<G>(d), kh.wn), dds = scaled(group_sum<G>(dd), kh.dhn);
+                const double d0 = group_sum<G>(d);
+                const double ds = scaled(d0 != 0.0, d0, kh.wn), dds = scaled(d0 != 0.0, group_sum<G>(dd), kh.dhn);
                 const double h3 = h * h * h;
                 const double f = ds * h3 - b;
                 const double df = dds * h3 + 3 * ds * (h * h);
@@ -352,34 +353,35 @@ __global__ void __launch_bounds__(PBLK, PRE_BLOCKS) k_pre(DevParams P, DevState 
             }
         }
         n_pairs += (unsigned)nn;
-        const double densS = scaled(group_sum<G>(dens), kh.wn);
         nn = group_sum<G>(nn);
+        const bool some = nn > 0;
+        const double densS = scaled(some, group_sum<G>(dens), kh.wn);
         vsig = group_max<G>(vsig);
         double dhdS = 0, niS = 0, presS = 0, dhpS = 0, dhnS = 0;
         if(disph) {
-            niS = scaled(group_sum<G>(ni), kh.wn);
-            presS = scaled(group_sum<G>(pres), kh.wn);
-            dhpS = scaled(group_sum<G>(dhp), kh.dhn);
-            dhnS = scaled(group_sum<G>(dhn), kh.dhn);
+            niS = scaled(some, group_sum<G>(ni), kh.wn);
+            presS = scaled(some, group_sum<G>(pres), kh.wn);
+            dhpS = scaled(some, group_sum<G>(dhp), kh.dhn);
+            dhnS = scaled(some, group_sum<G>(dhn), kh.dhn);
         } else if(!gsph) {
-            dhdS = scaled(group_sum<G>(dhd), kh.dhn);
+            dhdS = scaled(some, group_sum<G>(dhd), kh.dhn);
         }
         double divS = 0, rxS = 0, ryS = 0, rzS = 0;
         if(need_av) {
-            divS = scaled(group_sum<G>(divv), kh.dwn);
-            rxS = scaled(group_sum<G>(rx), kh.dwn);
-            ryS = scaled(group_sum<G>(ry), kh.dwn);
-            rzS = scaled(group_sum<G>(rz), kh.dwn);
+            divS = scaled(some, group_sum<G>(divv), kh.dwn);
+            rxS = scaled(some, group_sum<G>(rx), kh.dwn);
+            ryS = scaled(some, group_sum<G>(ry), kh.dwn);
+            rzS = scaled(some, group_sum<G>(rz), kh.dwn);
         }
         double gdS[3], guS[3], gvS[9];
         if(need_grad) {
 #pragma unroll
             for(int k = 0; k < 3; ++k) {
-                gdS[k] = scaled(group_sum<G>(gd[k]), kh.dwn);
-                guS[k] = scaled(group_sum<G>(gu[k]), kh.dwn);
+                gdS[k] = scaled(some, group_sum<G>(gd[k]), kh.dwn);
+                guS[k] = scaled(some, group_sum<G>(gu[k]), kh.dwn);
             }
 #pragma unroll
-            for(int k = 0; k < 9; ++k) gvS[k] = scaled(group_sum<G>(gv[k]), kh.dwn);
+            for(int k = 0; k < 9; ++k) gvS[k] = scaled(some, group_sum<G>(gv[k]), kh.dwn);
         }
 
         // ---- 3. epilogue (lane 0 of the group writes)
