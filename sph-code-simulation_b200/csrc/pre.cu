@@ -203,10 +203,11 @@ __global__ void __launch_bounds__(PBLK, PRE_BLOCKS) k_pre(DevParams P, DevState 
                         d += sb.w();
                         dd += sb.dh();
                     } else {
-                        d += pa.w * sa.w();
-                        dd += pa.w * sa.dh();
-                        d += pb.w * sb.w();
-                        dd += pb.w * sb.dh();
+                        const double ma = ia ? pa.w : 0.0, mb = ib ? pb.w : 0.0;
+                        d += ma * sa.w();
+                        dd += ma * sa.dh();
+                        d += mb * sb.w();
+                        dd += mb * sb.dh();
                     }
                 }
                 const double d0 = group_sum<G>(d);
@@ -274,7 +275,7 @@ __global__ void __launch_bounds__(PBLK, PRE_BLOCKS) k_pre(DevParams P, DevState 
             nn += q.in ? 1 : 0;
             const Shape<double, KER> sh(rT * kh.inv, q.in);
             const double w = sh.w();
-            const double mj = pj.w;
+            const double mj = q.in ? pj.w : 0.0;  // (a mass that is no number stays outside too)
             if(disph) {
                 const double dh = sh.dh();
                 const double uj = q.t.z;
