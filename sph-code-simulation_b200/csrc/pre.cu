@@ -272,6 +272,10 @@ __global__ void __launch_bounds__(PBLK, PRE_BLOCKS) k_pre(DevParams P, DevState 
         auto add = [&](const double4& pj, int j, const Pair& q) {
             double rT, rinvT;
             pair_distance(q.r2, rT, rinvT);
+            if(q.r2 < 0x1p-1000 && q.r2 > 0.0) {  // rare: v_sig needs v . r / r of these too
+                rinvT = rsqrt(q.r2);
+                rT = q.r2 * rinvT;
+            }
             nn += q.in ? 1 : 0;
             const Shape<double, KER> sh(rT * kh.inv, q.in);
             const double w = sh.w();
