@@ -106,6 +106,7 @@ struct sphgpu_ctx {
     int64_t relax_cap = 0;
     sphgpu::DevStatus* d_status = nullptr;
     sphgpu::DevStatus h_status{};
+    bool odd_box = false;            // DevStatus::odd_box of the current tree
 
     // learned Riemann guess (BF16 weights + FP32 biases on device)
     void* d_mlp = nullptr;            // BF16 / FP32 image read by the kernels

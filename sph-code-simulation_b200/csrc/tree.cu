@@ -84,7 +84,7 @@ __global__ void k_bbox_partial(const double4* __restrict__ pos, int n, double* _
 // One block reduces the partial boxes (one thread took 288 us for the 1,024
 // of a million particles).
 __global__ void __launch_bounds__(BLK) k_root(const double* __restrict__ part, int nparts, DevParams P,
-                                              double4* __restrict__ root)
+                                              double4* __restrict__ root, DevStatus* __restrict__ st)
 {
     __shared__ double s_box[BLK / 32][6];
     double lo[3], hi[3];
@@ -142,6 +142,8 @@ __global__ void __launch_bounds__(BLK) k_root(const double* __restrict__ part, i
         if(l < r) l = r;
     }
     *root = make_double4(c[0], c[1], c[2], l);
+    // squares of its lengths stay well inside FP32's range, or the walk scales them
+    if(!(l >= 0x1p-40 && l <= 0x1p60)) st->odd_box = 1;
 }
 
 // ---------------------------------------------------------------- keys
@@ -530,14 +532,14 @@ int tree_make(sphgpu_ctx* c)
     // root cube
     const int nb = (int)std::min<long long>(grid_for(n, BLK), 1024);
     int launches = 3;  // root, keys, levels
-    // node_pool, guard and nonfinite are adjacent words: clear all three, so an
-    // earlier "no free node" does not outlive a new upload
-    static_assert(offsetof(DevStatus, nonfinite) == offsetof(DevStatus, node_pool) + 2 * sizeof(int),
+    // node_pool, guard, nonfinite and odd_box are adjacent words: clear all four,
+    // so an earlier "no free node" does not outlive a new upload
+    static_assert(offsetof(DevStatus, odd_box) == offsetof(DevStatus, node_pool) + 3 * sizeof(int),
                   "status word layout");
-    SPHGPU_CUDA(c, cudaMemsetAsync(&c->d_status->node_pool, 0, 3 * sizeof(int), st));
+    SPHGPU_CUDA(c, cudaMemsetAsync(&c->d_status->node_pool, 0, 4 * sizeof(int), st));
     k_bbox_partial<<<nb, BLK, 0, st>>>(c->s.pos, n, c->d_bbox_part, c->d_status);
     ++launches;
-    k_root<<<1, BLK, 0, st>>>(c->d_bbox_part, nb, c->dp, c->d_root);
+    k_root<<<1, BLK, 0, st>>>(c->d_bbox_part, nb, c->dp, c->d_root, c->d_status);
     // keys + sort
     k_keys<<<grid_for(n, BLK), BLK, 0, st>>>(c->s.pos, n, c->d_root, D, c->d_keys, c->d_vals);
     launches += radix_sort(c->d_keys, c->d_vals, c->d_keys_alt, c->d_vals_alt, n, 3 * D, c->d_radix_scratch,
@@ -571,6 +573,7 @@ int tree_make(sphgpu_ctx* c)
         return fail(c, SPHGPU_ERR_NODE_POOL, "There is no free node.");
     }
     c->node_count = nnodes;
+    c->odd_box = c->h_status.odd_box != 0;
     // leaf order + permutation of the particle state
     k_leaf_order<<<grid_for(n, BLK), BLK, 0, st>>>(n, c->d_leaf_of_start, c->t.link, c->s.id, c->d_vals);
     k_permute<<<grid_for(n, BLK), BLK, 0, st>>>(n, c->d_vals, c->s, c->alt, c->prm.sph_type == SPHGPU_GSPH || c->prm.sph_type == SPHGPU_GDISPH ||

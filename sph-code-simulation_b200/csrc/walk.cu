@@ -34,6 +34,7 @@
 // buffer and re-runs (status.overflow).  More than neighbor_number * 1000
 // entries is the reference's fatal overflow (src/bhtree.cpp:129-135).
 #include <algorithm>
+#include <cfloat>
 #include <cmath>
 #include <cstddef>
 #include <cuda_runtime.h>
@@ -207,6 +208,15 @@ __device__ __forceinline__ unsigned hi32(f32x2 a) { return (unsigned)(a >> 32); 
 // mask << 1 | sign bit of v
 __device__ __forceinline__ unsigned sign_in(unsigned mask, unsigned v) { return __funnelshift_l(v, mask, 1); }
 
+// The power of two that brings `size` (where that is no positive finite number:
+// `other`, else 1) to 1 .. 2; below 2^-1022, to less.
+__device__ __forceinline__ double inverse_unit(double size, double other)
+{
+    if(!(size > 0.0 && size <= DBL_MAX)) size = other > 0.0 && other <= DBL_MAX ? other : 1.0;
+    const int e = max(__double2hiint(size) >> 20, 1);  // biased exponent
+    return __hiloint2double(max(2046 - e, 1) << 20, 0);
+}
+
 __device__ __forceinline__ double interval_gap(double c, double lo, double hi)
 {
     return c < lo ? lo - c : (c > hi ? c - hi : 0.0);
@@ -293,7 +303,12 @@ __global__ void __launch_bounds__(GW_WBLK) k_walk_windows(DevParams P, DevState 
 // The first `nsplit` blocks take the sub-groups of the split windows (32 items
 // per window, of which 32 / s are some), a warp each, beside the others, which
 // take a whole window per warp.
-template <bool IJ, int RES>
+// ODD (root boxes outside 2^-40 .. 2^60, whose squares leave FP32's range from
+// 2^64 on and the offsets themselves from 2^128 on): the classification runs in
+// the group's own unit, a power of two.  A form of its own, because scaling every
+// candidate costs an ordinary box 10 % (1.1 M sphere 3.35 -> 3.72 ms, 1 M shear
+// layer 2.97 -> 3.27).
+template <bool IJ, int RES, bool ODD>
 __global__ void __launch_bounds__(GW_WARPS * 32, RES) k_walk_group(DevParams P, DevState S, DevTree T, int n, int cap,
                                                              int* __restrict__ list, int* __restrict__ count,
                                                              DevStatus* __restrict__ st, double factor, int nsplit,
@@ -381,23 +396,26 @@ __global__ void __launch_bounds__(GW_WARPS * 32, RES) k_walk_group(DevParams P, 
         // in flight (1 M shear 3.33 -> 2.82 ms when it came; scalar FP32 3.01).
         const double cx = 0.5 * (blo[0] + bup[0]), cy = 0.5 * (blo[1] + bup[1]), cz = 0.5 * (blo[2] + bup[2]);
         const double ext_x = bup[0] - blo[0], ext_y = bup[1] - blo[1], ext_z = bup[2] - blo[2];
-        const float ax = (float)(xi - cx), ay = (float)(yi - cy), az = (float)(zi - cz);
+        const double unit = ODD ? inverse_unit(fmax(bext, IJ ? fmax(bh, T.ksize[0]) : bh), root.w) : 1.0;
+        const float ax = (float)((xi - cx) * unit), ay = (float)((yi - cy) * unit), az = (float)((zi - cz) * unit);
         bool wide = false;
         if(P.periodic) {
             wide = IJ || ext_x > P.range[0] - 2.02 * bh || ext_y > P.range[1] - 2.02 * bh
                 || ext_z > P.range[2] - 2.02 * bh;
         }
         const double image_err = wide ? 0x1p-21 * fmax(P.range[0], fmax(P.range[1], P.range[2])) : 0.0;
+        // (2^-120 and 2^-50: a radius below that lies in FP32's subnormals once
+        // squared, where errors are absolute: band pairs only)
         auto t_out = [&](double h) -> float {
-            const double t = h * (1.0 + 0x1p-20) + 0x1p-21 * bext + image_err;
-            return __double2float_ru(t * t * (1.0 + 0x1p-20));
+            const double t = (h * (1.0 + 0x1p-20) + 0x1p-21 * bext + image_err) * unit;
+            return __double2float_ru(t * t * (1.0 + 0x1p-20) + 0x1p-120);
         };
         auto t_in = [&](double h) -> float {
-            const double t = (h - delta - (0x1p-22 * bext + 0x1p-21 * h + image_err)) * (1.0 - 0x1p-20);
+            const double t = (h - delta - (0x1p-22 * bext + 0x1p-21 * h + image_err)) * (1.0 - 0x1p-20) * unit;
             // (a radius below about 2^-20 of the extent: band pairs only, so that
             // Tout < 2 t^2 wherever a pair may be taken without the exact test)
-            const double o = h * (1.0 + 0x1p-20) + 0x1p-21 * bext + image_err;
-            return t > 0.0 && o * o < 1.9 * (t * t) ? __double2float_rd(t * t * (1.0 - 0x1p-20)) : -1.0f;
+            const double o = (h * (1.0 + 0x1p-20) + 0x1p-21 * bext + image_err) * unit;
+            return t > 0x1p-50 && o * o < 1.9 * (t * t) ? __double2float_rd(t * t * (1.0 - 0x1p-20)) : -1.0f;
         };
         const float Ti_out = act ? t_out(hi) : -1.0f;
         const float Ti_in = act ? t_in(hi) : -1.0f;
@@ -410,7 +428,7 @@ __global__ void __launch_bounds__(GW_WARPS * 32, RES) k_walk_group(DevParams P, 
         const float gap = Ti_out - Ti_in;
         const f32x2 G2 = pack2(gap, gap);
         const float F_INF = __int_as_float(0x7f800000);
-        const float Lx = (float)P.range[0], Ly = (float)P.range[1], Lz = (float)P.range[2];
+        const float Lx = (float)(P.range[0] * unit), Ly = (float)(P.range[1] * unit), Lz = (float)(P.range[2] * unit);
 
         auto process = [&](int nproc) {
             // expand the queued nodes into their particles (warp prefix sum)
@@ -456,9 +474,9 @@ __global__ void __launch_bounds__(GW_WARPS * 32, RES) k_walk_group(DevParams P, 
                         tko = t_out(ks);
                         tki = t_in(ks);
                     }
-                    fx = (float)bx;
-                    fy = (float)by;
-                    fz = (float)bz;
+                    fx = (float)(bx * unit);
+                    fy = (float)(by * unit);
+                    fz = (float)(bz * unit);
                     s_cpos[w][lane] = make_double4(pj.x, pj.y, pj.z, ks);
                     s_cid[w][lane] = q;
                 }
@@ -737,8 +755,9 @@ int run_walk(sphgpu_ctx* c, int which, bool guess, double ratio, bool exhaustive
             k_walk_windows<<<grid_for(n, GW_WBLK), GW_WBLK, 0, st>>>(c->dp, c->s, n, which == 0 && guess ? 1 : 0, ratio,
                                                                      which == 0 ? sk : SkinOut{1.0, nullptr, nullptr},
                                                                      c->d_status, width, c->d_split);
-            auto* k = which == 0 ? (few ? k_walk_group<false, 8> : k_walk_group<false, 10>)
-                                 : (few ? k_walk_group<true, 8> : k_walk_group<true, 10>);
+            auto* k = which == 0 ? (few ? k_walk_group<false, 8, false> : k_walk_group<false, 10, false>)
+                                 : (few ? k_walk_group<true, 8, false> : k_walk_group<true, 10, false>);
+            if(c->odd_box) k = which == 0 ? k_walk_group<false, 8, true> : k_walk_group<true, 8, true>;
             k<<<nsplit + grid, GW_WARPS * 32, 0, st>>>(c->dp, c->s, c->t, n, (int)cap, list, count, c->d_status,
                                                        which == 0 && guess ? sk.factor : 1.0, nsplit, width,
                                                        c->d_split);
@@ -751,10 +770,10 @@ int run_walk(sphgpu_ctx* c, int which, bool guess, double ratio, bool exhaustive
                                                            c->d_status, 0, 1.0, SkinOut{1.0, nullptr, nullptr});
         }
         SPHGPU_LAUNCH_CHECK(c, "neighbour walk");
-        // the first eight status words: the walk's own and the pass guard of
+        // the first nine status words: the walk's own and the pass guard of
         // the bottom-up mass pass that ran before it
-        static_assert(offsetof(DevStatus, pass_guard) == 7 * sizeof(int), "status word layout");
-        SPHGPU_CUDA(c, cudaMemcpyAsync(&c->h_status, c->d_status, 8 * sizeof(int), cudaMemcpyDeviceToHost, st));
+        static_assert(offsetof(DevStatus, pass_guard) == 8 * sizeof(int), "status word layout");
+        SPHGPU_CUDA(c, cudaMemcpyAsync(&c->h_status, c->d_status, 9 * sizeof(int), cudaMemcpyDeviceToHost, st));
         SPHGPU_CUDA(c, cudaStreamSynchronize(st));
         if(c->h_status.fatal) {
             return fail(c, SPHGPU_ERR_NEIGHBOR_OVERFLOW,
