@@ -91,7 +91,8 @@ struct DevStatus {
     int node_pool;         // node pool exhausted
     int guard;             // a neighbour walk hit its node-count bound (corrupt tree)
     int nonfinite;         // a particle position is NaN or infinite
-    int odd_box;           // the root box is out of the range of the walk's ordinary FP32 form
+    int odd_box;           // the walk's ordinary FP32 form does not hold: the root box is out of
+                           // its range, or a particle lies outside the periodic box
     int pass_guard;        // PASS_GUARD_* bits: a bottom-up pass or gravity walk hit its bound
     unsigned long long newton_nonconv;
     unsigned long long riemann_solves;

@@ -160,12 +160,16 @@ __device__ __forceinline__ double child_center(double c, int bit, double e)
 }
 
 __global__ void k_keys(const double4* __restrict__ pos, int n, const double4* __restrict__ root, int depth,
-                       uint64_t* __restrict__ keys, uint32_t* __restrict__ vals)
+                       uint64_t* __restrict__ keys, uint32_t* __restrict__ vals, DevParams P,
+                       DevStatus* __restrict__ st)
 {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if(i >= n) return;
     const double4 p = pos[i];
     const double4 r = *root;
+    if(P.periodic && (p.x < P.lo[0] || p.x > P.hi[0] || p.y < P.lo[1] || p.y > P.hi[1] || p.z < P.lo[2] || p.z > P.hi[2])
+       && *reinterpret_cast<volatile int*>(&st->odd_box) == 0)
+        st->odd_box = 1;
     double cx = r.x, cy = r.y, cz = r.z, e = r.w;
     uint64_t key = 0;
     for(int l = 0; l < depth; ++l) {
@@ -541,7 +545,8 @@ int tree_make(sphgpu_ctx* c)
     ++launches;
     k_root<<<1, BLK, 0, st>>>(c->d_bbox_part, nb, c->dp, c->d_root, c->d_status);
     // keys + sort
-    k_keys<<<grid_for(n, BLK), BLK, 0, st>>>(c->s.pos, n, c->d_root, D, c->d_keys, c->d_vals);
+    k_keys<<<grid_for(n, BLK), BLK, 0, st>>>(c->s.pos, n, c->d_root, D, c->d_keys, c->d_vals, c->dp,
+                                             c->d_status);
     launches += radix_sort(c->d_keys, c->d_vals, c->d_keys_alt, c->d_vals_alt, n, 3 * D, c->d_radix_scratch,
                            &c->d_status->pass_guard, st);
     // nodes

@@ -305,9 +305,10 @@ __global__ void __launch_bounds__(GW_WBLK) k_walk_windows(DevParams P, DevState 
 // take a whole window per warp.
 // ODD (root boxes outside 2^-40 .. 2^60, whose squares leave FP32's range from
 // 2^64 on and the offsets themselves from 2^128 on): the classification runs in
-// the group's own unit, a power of two.  A form of its own, because scaling every
-// candidate costs an ordinary box 10 % (1.1 M sphere 3.35 -> 3.72 ms, 1 M shear
-// layer 2.97 -> 3.27).
+// the group's own unit, a power of two; and particles outside the periodic box,
+// which an offset's one image may not bring near: the exact test decides those
+// pairs.  A form of its own, because both for every candidate cost an ordinary box
+// 10 % (1.1 M sphere 3.35 -> 3.72 ms, 1 M shear layer 2.97 -> 3.27).
 template <bool IJ, int RES, bool ODD>
 __global__ void __launch_bounds__(GW_WARPS * 32, RES) k_walk_group(DevParams P, DevState S, DevTree T, int n, int cap,
                                                              int* __restrict__ list, int* __restrict__ count,
@@ -465,6 +466,9 @@ __global__ void __launch_bounds__(GW_WARPS * 32, RES) k_walk_group(DevParams P, 
                 if(have) {
                     const double ks = IJ ? __ldg(&T.pks[q]) : 0.0;
                     double bx = xsub(pj.x, cx), by = xsub(pj.y, cy), bz = xsub(pj.z, cz);
+                    [[maybe_unused]] const bool far = ODD && wide
+                        && (fabs(bx) + 0.5 * ext_x > 1.5 * P.range[0] || fabs(by) + 0.5 * ext_y > 1.5 * P.range[1]
+                            || fabs(bz) + 0.5 * ext_z > 1.5 * P.range[2]);
                     if(P.periodic) {
                         bx = min_image(bx, P.range[0]);
                         by = min_image(by, P.range[1]);
@@ -477,6 +481,7 @@ __global__ void __launch_bounds__(GW_WARPS * 32, RES) k_walk_group(DevParams P, 
                     fx = (float)(bx * unit);
                     fy = (float)(by * unit);
                     fz = (float)(bz * unit);
+                    if(ODD && far) fx = __int_as_float(0x7fffffff);  // NaN: in the band of every lane
                     s_cpos[w][lane] = make_double4(pj.x, pj.y, pj.z, ks);
                     s_cid[w][lane] = q;
                 }
