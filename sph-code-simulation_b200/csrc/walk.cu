@@ -495,7 +495,7 @@ __global__ void __launch_bounds__(GW_WARPS * 32, RES) k_walk_group(DevParams P, 
                 }
                 __syncwarp();
                 unsigned in_mask = 0u;
-                if(act) {
+                if(act && (!IJ || hi == hi)) {  // (no pair lies within a NaN radius)
                     unsigned band_mask = 0u;
                     if(!IJ && !wide) {
                         unsigned near = 0u, inside = 0u;
