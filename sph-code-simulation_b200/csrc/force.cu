@@ -92,7 +92,8 @@ __device__ __forceinline__ T vl_newton_step(T p, T ul, T pl, T vl, T cl, T ur, T
 }
 
 // The same update and the final u* in FP64 with an operation policy
-// (rounded.cuh); every quotient and root is rounded as the general operations'.
+// (rounded.cuh): quotients and roots rounded as the general operations', but for
+// the rare operands named there.
 template <typename Op>
 __device__ __forceinline__ double vl_step(Op& op, double p, double ul, double pl, double vl, double cl, double ur,
                                           double pr, double vr, double cr, double g1, double g2)

@@ -79,7 +79,7 @@ __device__ __forceinline__ void hk_fg_rn(double r, double rinv, double r3, doubl
     const double p = near ? (1.0 / 3.0 - t) + w : (4.0 / 3.0 - u + t) - w;
     const double fe = quot_rn((near ? -0.5 : -1.0) * u * u * p + (near ? 1.4 : 1.6), k.x, k.z);
     const double r15 = 15 * r;
-    const double fm = -recip_rn(r15, rinv * (1.0 / 15.0)) + fe;
+    const double fm = -recip_any(r15, rinv * (1.0 / 15.0)) + fe;
     const double gn = 4.0 / 3.0 - 1.2 * u * u + 0.5 * u * u * u;
     const double gm = -1.0 / 15 + 8.0 / 3 * u * u * u - 3.0 * u * u * u * u + 1.2 * u * u * u * u * u
         - quot_rn(u3 * u * u * u, 6.0, 1.0 / 6.0);
@@ -97,7 +97,8 @@ __global__ void k_half(DevState S, int n, double4* __restrict__ half)
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if(i >= n) return;
     const double h = S.vel[i].w, e = h * 0.5, e3 = e * e * e;
-    half[i] = pair_range(h) ? make_double4(e, e3, recip_rn(e), recip_rn(e3)) : make_double4(-1.0, 0.0, 0.0, 0.0);
+    half[i] = pair_range(h) && !all_ones(e) && !all_ones(e3) ? make_double4(e, e3, recip_rn(e), recip_rn(e3))
+                                                             : make_double4(-1.0, 0.0, 0.0, 0.0);
 }
 
 // subset != null: only the listed particles (the mixed form's FP64
@@ -170,7 +171,7 @@ __global__ void __launch_bounds__(GBLK, RES) k_gravity(DevParams P, DevState S, 
         if(!open) {
             ++n_mono;
             double rinv;
-            if(mid_range(d2)) {
+            if(mid_range(d2) && root_not_ones(d2)) {
                 const double y = rsqrt_near(d2);
                 rinv = recip_rn(root_rn(d2, y), y);
             } else {
@@ -191,12 +192,12 @@ __global__ void __launch_bounds__(GBLK, RES) k_gravity(DevParams P, DevState S, 
                 const Vec3d r = offset(pq);
                 const double r2 = r.x * r.x + r.y * r.y + r.z * r.z;
                 double f1, f2, g1, g2;
-                if(pair_range(r2) && ki.x > 0.0 && kq.x > 0.0) {
+                if(pair_range(r2) && root_not_ones(r2) && ki.x > 0.0 && kq.x > 0.0) {
                     const double y = rsqrt_near(r2);
                     const double rr = root_rn(r2, y);
                     const double rinv = recip_rn(rr, y);
                     const double r3 = rr * rr * rr;
-                    const double r3i = recip_rn(r3, y * y * y);
+                    const double r3i = recip_any(r3, y * y * y);
                     hk_fg_rn(rr, rinv, r3, r3i, ki, f1, g1);
                     hk_fg_rn(rr, rinv, r3, r3i, kq, f2, g2);
                 } else {

@@ -11,6 +11,15 @@
 // step of the Taylor series of 1 / sqrt(1 - e) and 1 / (1 - e).  The fused
 // operations are explicit, so the files built without contraction keep every
 // other operation as written.
+//
+// What the method gives: roots and reciprocals of an approximation within a unit
+// in the last place are rounded, a reciprocal's divisor with a significand of all
+// ones excepted (all_ones below); quotients need the rounded reciprocal.  Quick's
+// div and div0 take one that is good to about an ulp: theirs are the rounded
+// quotients but for operands whose quotient lies next to the middle of two doubles
+// (2 in 10^8 of the nearest there are, none of 10^9 random ones), or a unit off
+// for a divisor of all ones.  tests/cpp/rounded_ops.cu counts all of them against
+// CUDA's operations.
 #pragma once
 
 namespace sphgpu {
@@ -22,6 +31,17 @@ __device__ __forceinline__ bool mid_range(double x)
     const unsigned hi = (unsigned)__double2hiint(x) & 0x7fffffffu;
     return hi - ((1023u - 300u) << 20) < (600u << 20);
 }
+
+// True for a significand of all ones, the one exception of the reciprocal's
+// correction: 1 / b then lies just above the middle of a power of two and the
+// next double, and a y of that power ties down to itself.
+__device__ __forceinline__ bool all_ones(double x)
+{
+    return (unsigned)__double2loint(x) == 0xffffffffu && ((unsigned)__double2hiint(x) | 0xfff00000u) == 0xffffffffu;
+}
+// False for the few positive a (and others, one in 2^31) whose rounded root is a
+// power of two less one unit in the last place, a significand of all ones.
+__device__ __forceinline__ bool root_not_ones(double a) { return (unsigned)__double2loint(a) < 0xfffffffeu; }
 
 __device__ __forceinline__ double rsqrt_seed(double a)
 {
@@ -63,6 +83,14 @@ __device__ __forceinline__ double recip_rn(double b)
     return recip_rn(b, __fma_rn(y, __fma_rn(e, e, e), y));
 }
 
+// 1 / b, rounded, from a y a few units off (corrected twice) and for a significand
+// of all ones too: the double after the power of two
+__device__ __forceinline__ double recip_any(double b, double y)
+{
+    const double r = recip_rn(b, recip_rn(b, y));
+    return __hiloint2double(__double2hiint(r), __double2loint(r) | (all_ones(b) ? 1 : 0));
+}
+
 // a / b, rounded, from y = 1 / b rounded
 __device__ __forceinline__ double quot_rn(double a, double b, double y)
 {
@@ -73,9 +101,10 @@ __device__ __forceinline__ double quot_rn(double a, double b, double y)
 // Quotients and roots of one pair: Quick takes the forms above and notes when a
 // result may have left the range where they hold (its pair is then computed
 // again with Ieee); no branch in between, so independent operations overlap.
-// A result in 2^-400 .. 2^400 is the rounded one: an operand outside the
-// exponent range yields zero, infinity or NaN, and a residual that lost bits to
-// underflow needs operands below 2^-900.
+// A result in 2^-400 .. 2^400 then holds as above: an operand outside the
+// exponent range yields zero, infinity or NaN.  (Operands below 2^-900 with such a
+// quotient are not flagged: their residual may lose bits, and the result its
+// last.)
 struct Ieee {
     static constexpr bool quick = false;
     bool bad = false;
