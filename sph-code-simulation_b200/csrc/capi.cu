@@ -225,7 +225,9 @@ int alloc_all(sphgpu_ctx* c, int n)
        || (rc = dalloc(c, c->t.counter, nc)) || (rc = dalloc(c, c->t.nnodes, 4))
        || (rc = dalloc(c, c->t.leaf_of, n)) || (rc = dalloc(c, c->t.pks, n)))
         return rc;
-    if(c->prm.use_gravity && (rc = dalloc(c, c->d_half, n))) return rc;
+    // the FP64 walk's half kernels: also of the mixed form's FP64 re-evaluation
+    const bool walk64 = c->prm.use_gravity && (c->prm.precision != SPHGPU_MIXED || c->prm.mixed_acc_tol > 0.0);
+    if(walk64 && (rc = dalloc(c, c->d_half, n))) return rc;
     if((rc = dalloc(c, c->d_root, 1)) || (rc = dalloc(c, c->d_bbox_part, 6 * 1024)) || (rc = dalloc(c, c->d_keys, n))
        || (rc = dalloc(c, c->d_keys_alt, n)) || (rc = dalloc(c, c->d_vals, n)) || (rc = dalloc(c, c->d_vals_alt, n))
        || (rc = dalloc(c, c->d_nstart, n)) || (rc = dalloc(c, c->d_base, n)) || (rc = dalloc(c, c->d_lvl, n))
