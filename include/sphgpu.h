@@ -392,11 +392,12 @@ int sphgpu_get_stage_times(sphgpu_ctx* ctx, double* ms /* [SPHGPU_NSTAGES] */,
    hit since the last wait by a device pass that runs without a host wait of
    its own: the bottom-up mass and kernel_size passes and the gravity walks,
    which bound their loops by the tree depth and node count instead of
-   looping on a corrupt tree.  sphgpu_integrate, sphgpu_initialize and the
+   looping on a corrupt tree, and the key sort, whose tiles count their waits
+   for one another.  sphgpu_integrate, sphgpu_initialize and the
    next tree_make / neighbour walk report it the same way. */
 int sphgpu_synchronize(sphgpu_ctx* ctx);
 /* Test hook: set PASS_GUARD bits (1 mass, 2 set_kernel, 4 gravity, 8 mixed
-   gravity) on the device as those passes do when they hit their bound, so a
+   gravity, 16 key sort) on the device as those passes do when they hit their bound, so a
    test can check that the next synchronising call reports it without
    corrupting a tree.  No counterpart in the reference. */
 int sphgpu_test_flag_pass_guard(sphgpu_ctx* ctx, int bits);

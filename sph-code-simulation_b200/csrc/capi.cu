@@ -1204,7 +1204,7 @@ int sphgpu_synchronize(sphgpu_ctx* c)
 
 int sphgpu_test_flag_pass_guard(sphgpu_ctx* c, int bits)
 {
-    if(!c || !c->d_status || bits <= 0 || bits > 15) return SPHGPU_ERR_ARG;
+    if(!c || !c->d_status || bits <= 0 || bits > 31) return SPHGPU_ERR_ARG;
     SPHGPU_CUDA(c, cudaMemcpyAsync(&c->d_status->pass_guard, &bits, sizeof(int), cudaMemcpyHostToDevice, c->stream));
     SPHGPU_CUDA(c, cudaStreamSynchronize(c->stream));
     return SPHGPU_OK;
