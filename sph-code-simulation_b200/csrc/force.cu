@@ -698,7 +698,7 @@ __device__ __forceinline__ void iterate_star(Op& op, const double* L, const doub
 // Measured (general operations, kernel function at run time -> now): 1.1 M disph
 // sphere 2.84 -> 1.82 ms (41 % of the issue slots before, FP64 pipe 45 %), 1 M
 // shear layer 3.07 -> 1.99, 0.49 M ssph sphere 0.60 -> 0.36, 17 K 0.042 -> 0.024,
-// 244 K gdisph tube 0.97 -> 0.68, 2 M gsph tube 8.4 -> 6.4 (FP64 pipe 50 %).
+// 244 K gdisph tube 0.97 -> 0.68, 2 M gsph tube 8.4 -> 6.4 (FP64 pipe 52 % at 245 K).
 template <int G, int TYPE, int KER, bool PER, int MODE>
 __global__ void __launch_bounds__(force64_threads(TYPE), force64_blocks(TYPE)) k_force64(DevParams P, DevState S, int n, const int* __restrict__ list,
                                                 const int* __restrict__ count, int cap, const double* __restrict__ dtp,

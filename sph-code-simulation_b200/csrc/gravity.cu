@@ -19,8 +19,8 @@
 // reference's on the same tree.  The mixed-precision walk is in
 // gravity_mixed.cu (compiled with FMA contraction).
 //
-// What bounds it: issue slots and the FP64 pipe (1.1 M sphere: 66 % of the
-// issue slots, FP64 pipe 57 %, 17 of 32 lanes per instruction).  An accepted
+// What bounds it: issue slots and the FP64 pipe (0.56 M sphere: 66 % of the
+// issue slots, FP64 pipe 58 %, 17 of 32 lanes per instruction).  An accepted
 // node needs 1 / sqrt(d2) with both operations rounded as the reference's, an
 // opened leaf a pair of spline kernels with ten quotients, on the few lanes
 // that open one while the warp waits.  The roots and quotients are taken with
@@ -28,8 +28,9 @@
 // the chains of one term overlap, and quotients by h / 2 and its cube share
 // one reciprocal per particle (k_half).  Measured (fixed state, one box, the
 // general operations -> these): 17 K sphere 0.945 -> 0.52 ms, 137 K 2.00 ->
-// 1.38, 1.1 M 13.2 -> 9.9, 4.2 M 47.7 -> 37.5; without the softened pairs'
-// arithmetic 7.3 ms on the 1.1 M sphere (timing-only copy).
+// 1.38, 1.1 M 13.2 -> 9.9, 4.2 M 47.7 -> 37.5; then 1 - 3 % more (1.1 M 10.1) for the
+// divisors of all ones; without the softened pairs' arithmetic 7.3 ms on the 1.1 M
+// sphere (timing-only copy).
 // Measured and not kept (1.1 M sphere, against 9.9 ms): each lane's
 // interactions queued in shared memory and summed a queue at a time, walk test
 // in FP32 (13.2 ms; the queueing costs as many instructions as it aligns);

@@ -535,9 +535,9 @@ __global__ void __launch_bounds__(PBLK, PRE_BLOCKS) k_pre_mixed(DevParams P, Dev
         // the candidates within (1 + 4e-4) h in a scratch row; after a
         // converged sweep (|h_new - h| < 1e-4 (h_new + h), so h_new <
         // (1 + 2.0003e-4) h) they hold every pair of the fused pass, which
-        // then reads them instead of the whole list (8.78 M sphere: pre 31.8
-        // -> 30.8 ms FP64, 27.4 -> 24.1 ms FP32; the gsph and gdisph bodies
-        // spill with it and run slower)
+        // then reads them instead of the whole list (8.78 M sphere, when it
+        // came: 27.4 -> 24.1 ms, now 22.1; the gsph and gdisph bodies spilled
+        // with it and ran slower)
         constexpr bool keep = TYPE == SPHGPU_DISPH;
         int* srow = scratch + (size_t)(valid ? i : 0) * (size_t)scap;
         int nk = 0;

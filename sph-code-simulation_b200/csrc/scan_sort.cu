@@ -6,7 +6,9 @@
 // pass is one kernel that reads and writes every key and value once.  A tile
 // (2048 keys) ranks its keys stably (warp match + per-warp counts), learns the
 // counts of the tiles before it by decoupled look-back (D. Merrill and M.
-// Garland, "Single-pass parallel prefix scan with decoupled look-back", 2016),
+// Garland, "Single-pass parallel prefix scan with decoupled look-back", 2016; one
+// histogram read and one look-back kernel per digit is the sort of A. Adinets and
+// D. Merrill, "Onesweep: a faster least significant digit radix sort for GPUs", 2022),
 // stages its keys digit-contiguously in shared memory and writes them so that
 // consecutive threads store consecutive addresses.
 // Below about 200 K keys a pass is bound by launches and the latency of the

@@ -385,7 +385,7 @@ __global__ void __launch_bounds__(GW_WARPS * 32, RES) k_walk_group(DevParams P, 
         // L/2 - ext/2 > h on every axis the pair is then outside either way
         // (|d| > L/2 > h, and its nearest image is L/2 - ext/2 away or more) and
         // nothing need be done.  Otherwise (`wide`: a thin box) each lane takes
-        // the nearest image in FP32, which costs E another 2^-22 L.  (Candidates
+        // the nearest image in FP32, which costs E another 2^-21 L.  (Candidates
         // that might have another image used to run the exact test for every
         // lane: 131 K shear layer 1.31 ms, 245 K tube 1.44 ms, now 0.64 and 0.61.)
         // Each lane classifies a chunk of 32 staged candidates branch-free into
